@@ -1030,6 +1030,19 @@ void build_tu_coeffs(amg_ctx* ctx, cudaStream_t s) {
     build_scaled_coeffs<R>(ctx, s);
 }
 
+// Blocks of k_tu_stored per SM.  In FP32 9 blocks fit an SM (54 registers),
+// and a grid that fills them all leaves no room for the PME chain's blocks
+// beside it until its last wave: with 6 striding blocks the chain runs
+// through (32,768 waters: 3.67 -> 3.54 ms per evaluation; 4 blocks 3.58, 8
+// blocks 3.61; 4,096 waters: level).  In FP64 (64 registers) the full grid is
+// the faster one (8,000 waters: 2.00 against 2.03 ms).
+template <class R>
+unsigned tu_blocks(const amg_ctx* ctx, int lanes) {
+    constexpr int kTuBlocks = 6;
+    const unsigned all = nblk((size_t)ctx->n * lanes);
+    return sizeof(R) == 4 ? std::min(all, (unsigned)ctx->num_sms * kTuBlocks) : all;
+}
+
 // A v with the stored coefficients; v4 is the R4 copy of (vd, vp).  With
 // vAv (Ewald only) the dot products v.Av are added to vAv[0..1].  `apart`
 // (Ewald, with vAv) keeps the real-space field out of Ad, Ap: the gather then
@@ -1044,7 +1057,7 @@ void matvec_stored(amg_ctx* ctx, cudaStream_t s, const R4<R>* v4, const double* 
     // real space on the side stream, PME on s
     cudaStream_t r = ctx->ewald ? fork_side(ctx, s) : s;
     LPA_DISPATCH(ctx->lpa, {
-        k_tu_stored<R, L><<<nblk((size_t)n * L), kThreads, 0, r>>>(n, ctx->sids, ctx->cnb, A.c0, ctx->cap, ctx->nnb, ctx->xoff,
+        k_tu_stored<R, L><<<tu_blocks<R>(ctx, L), kThreads, 0, r>>>(n, ctx->sids, ctx->cnb, A.c0, ctx->cap, ctx->nnb, ctx->xoff,
                                                                     v4, ctx->Fd, ctx->Fp, apart ? vd : nullptr,
                                                                     apart ? vp : nullptr, apart ? vAv : nullptr);
     });
@@ -1954,15 +1967,18 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     ctx->usolvcut = std::min(P->usolvcut, P->cutoff);
     ctx->cell_shape = P->cell_shape;
     for (int a = 0; a < 3; a++) ctx->K[a] = P->nfft[a];
-    // the solve's streams at the highest priority, the permanent-multipole
-    // force stream at the lowest: its blocks fill what the solve leaves idle
+    // the main streams (the PME chains, the PCG vectors) at the highest
+    // priority: their kernels are short and each waits for the last, so they
+    // go before the long pair kernels of the side streams (one step lower);
+    // the permanent-multipole force stream at the lowest: its blocks fill what
+    // the solve leaves idle
     int plo = 0, phi = 0;
     CK(cudaDeviceGetStreamPriorityRange(&plo, &phi));
-    const int pmain = phi;
+    const int pmain = phi, pside = std::min(plo, phi + 1);
     CK(cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, pmain));
     CK(cudaStreamCreateWithPriority(&ctx->st2, cudaStreamNonBlocking, pmain));
     for (int k = 0; k < 3; k++) {
-        CK(cudaStreamCreateWithPriority(&ctx->side[k], cudaStreamNonBlocking, k == kMpoleSide ? plo : pmain));
+        CK(cudaStreamCreateWithPriority(&ctx->side[k], cudaStreamNonBlocking, k == kMpoleSide ? plo : pside));
         CK(cudaEventCreateWithFlags(&ctx->efork[k], cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&ctx->ejoin[k], cudaEventDisableTiming));
     }
@@ -2739,11 +2755,11 @@ int amg_time_tu_kernel(amg_ctx* ctx, int32_t reps, int64_t flush_bytes, double* 
             CK(cudaEventRecord(a, ctx->st));
             LPA_DISPATCH(ctx->lpa, {
                 if (mixed)
-                    k_tu_stored<float, L><<<nblk((size_t)n * L), kThreads, 0, ctx->st>>>(
+                    k_tu_stored<float, L><<<tu_blocks<float>(ctx, L), kThreads, 0, ctx->st>>>(
                         n, ctx->sids, ctx->cnb, ctx->af.c0, ctx->cap, ctx->nnb, ctx->xoff, ctx->af.p4,
                         ctx->Fd, ctx->Fp);
                 else
-                    k_tu_stored<double, L><<<nblk((size_t)n * L), kThreads, 0, ctx->st>>>(
+                    k_tu_stored<double, L><<<tu_blocks<double>(ctx, L), kThreads, 0, ctx->st>>>(
                         n, ctx->sids, ctx->cnb, ctx->ad.c0, ctx->cap, ctx->nnb, ctx->xoff, ctx->ad.p4,
                         ctx->Fd, ctx->Fp);
             });

@@ -398,6 +398,8 @@ __global__ void __launch_bounds__(128) k_tu_coeffs(int n, const int* __restrict_
 // slots plus the site's scaled partners.  u4: [n][2] R4 in cell order.
 // With vAv, also adds -v.F of both sets to vAv[0..1] (the real-space share
 // of v.Av when the rest of Av is assembled apart, see k_gather_field).
+// Bound by the L1 pipe and HBM (20 B streamed and 32 B gathered per pair).
+// Blocks stride over the sites: see tu_blocks for the grid.
 template <class R, int LPA>
 __global__ void __launch_bounds__(128) k_tu_stored(int n, const int* __restrict__ order, const int* __restrict__ cnb,
                                                    const R4<R>* __restrict__ c0, int cap,
@@ -406,21 +408,24 @@ __global__ void __launch_bounds__(128) k_tu_stored(int n, const int* __restrict_
                                                    double* __restrict__ Fp, const double* __restrict__ vd = nullptr,
                                                    const double* __restrict__ vp = nullptr,
                                                    double* __restrict__ vAv = nullptr) {
-    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPA, lane = threadIdx.x % LPA;
-    const int gs = min(g, n - 1), i = order[gs];  // gs: the site's position in cell order
-    const int cnt = g < n ? nnb[i] + (xoff[i + 1] - xoff[i]) : 0;
-    const size_t base = (size_t)i * cap;
-    R ax = 0, ay = 0, az = 0, bx_ = 0, by = 0, bz = 0;
-    row_apply<R, LPA, sizeof(R) == 4 ? 4 : 2>(cnb, c0, base, cnt, lane, gs, u4, ax, ay, az, bx_, by, bz);
-    double sx = group_sum<LPA>((double)ax), sy = group_sum<LPA>((double)ay), sz = group_sum<LPA>((double)az);
-    double tx = group_sum<LPA>((double)bx_), ty = group_sum<LPA>((double)by), tz = group_sum<LPA>((double)bz);
+    const int lane = threadIdx.x % LPA, per_block = blockDim.x / LPA;
     double dd = 0, dp = 0;
-    if (lane == 0 && g < n) {
-        Fd[3 * i] = sx; Fd[3 * i + 1] = sy; Fd[3 * i + 2] = sz;
-        Fp[3 * i] = tx; Fp[3 * i + 1] = ty; Fp[3 * i + 2] = tz;
-        if (vAv) {  // this part's share of v.Av (Av holds -F)
-            dd = -(vd[3 * i] * sx + vd[3 * i + 1] * sy + vd[3 * i + 2] * sz);
-            dp = -(vp[3 * i] * tx + vp[3 * i + 1] * ty + vp[3 * i + 2] * tz);
+    for (int g0 = blockIdx.x * per_block; g0 < n; g0 += gridDim.x * per_block) {
+        const int g = g0 + threadIdx.x / LPA;
+        const int gs = min(g, n - 1), i = order[gs];  // gs: the site's position in cell order
+        const int cnt = g < n ? nnb[i] + (xoff[i + 1] - xoff[i]) : 0;
+        const size_t base = (size_t)i * cap;
+        R ax = 0, ay = 0, az = 0, bx_ = 0, by = 0, bz = 0;
+        row_apply<R, LPA, sizeof(R) == 4 ? 4 : 2>(cnb, c0, base, cnt, lane, gs, u4, ax, ay, az, bx_, by, bz);
+        double sx = group_sum<LPA>((double)ax), sy = group_sum<LPA>((double)ay), sz = group_sum<LPA>((double)az);
+        double tx = group_sum<LPA>((double)bx_), ty = group_sum<LPA>((double)by), tz = group_sum<LPA>((double)bz);
+        if (lane == 0 && g < n) {
+            Fd[3 * i] = sx; Fd[3 * i + 1] = sy; Fd[3 * i + 2] = sz;
+            Fp[3 * i] = tx; Fp[3 * i + 1] = ty; Fp[3 * i + 2] = tz;
+            if (vAv) {  // this part's share of v.Av (Av holds -F)
+                dd -= vd[3 * i] * sx + vd[3 * i + 1] * sy + vd[3 * i + 2] * sz;
+                dp -= vp[3 * i] * tx + vp[3 * i + 1] * ty + vp[3 * i + 2] * tz;
+            }
         }
     }
     if (vAv) {
