@@ -771,7 +771,13 @@ void enqueue_lists(amg_ctx* ctx, cudaStream_t s) {
         // decided by the FP64 image of the cell)
         auto kern = cg.general ? k_neighbors_cells<true> : cg.centred ? k_neighbors_cells<false, true>
                                                                       : k_neighbors_cells<false>;
-        kern<<<(unsigned)ncell, kNbrThreads, 0, s>>>(ctx->spos, ctx->sids, ctx->cstart, ctx->cend, cg, ctx->bx, cut2,
+        // with fewer than 4 cells per SM, two blocks per cell: the last wave
+        // is then short (4,096 waters, 343 cells: 891 -> 879 us per
+        // evaluation; 13,824 waters at 9 A, 512 cells: 513 -> 495 us; more
+        // blocks repeat the staging for nothing: 1,500 waters, 125 cells: 642
+        // us with 2, 650 with 5)
+        const unsigned split = ncell < 4 * (size_t)ctx->num_sms ? 2 : 1;
+        kern<<<dim3((unsigned)ncell, split), kNbrThreads, 0, s>>>(ctx->spos, ctx->sids, ctx->cstart, ctx->cend, cg, ctx->bx, cut2,
                                                      1e-3 * cut2, ctx->cap, ctx->xoff, ctx->xidx, ctx->xrange, ctx->nbr,
                                                      ctx->cnb, ctx->nnb, ctx->overflow);
     } else {

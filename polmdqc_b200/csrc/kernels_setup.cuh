@@ -288,9 +288,15 @@ __global__ void k_neighbors(int n, const double4* __restrict__ spos, const unsig
 // order, each in sorted order), so the rows are identical too.  Staging is
 // chunked (kNbrChunk candidates, kNbrHome home atoms at a time), so any cell
 // occupancy works.
+//
+// Bound by instruction issue: ~1,200 candidates per site at a 7 A cutoff, of
+// which 12% are partners.  So a warp (one home site) only tests distances in
+// its scan and queues the hits; the queue is decided (near the cutoff, scaled
+// partners) and written 32 at a time with full lanes.
 constexpr int kNbrChunk = 1280;
 constexpr int kNbrHome = 128;
 constexpr int kNbrThreads = 256;
+constexpr int kNbrScan = 4;  // candidates per lane and scan step: loads and tests in flight together
 
 // CENTRED (truncated octahedron, rhombic dodecahedron): the stencil is the 27
 // cells around the home cell plus the 27 around the cell half a prism away,
@@ -314,12 +320,14 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_cells(
     __shared__ float4 hpos[kNbrHome];
     __shared__ int hid[kNbrHome], hx0[kNbrHome], hx1[kNbrHome];
     __shared__ int2 hxr[kNbrHome];
-    __shared__ int rstart[54], rpre[55];
+    __shared__ int rstart[54], rpre[64];  // rpre: first candidate of each stencil cell, then the total to the end
+    __shared__ unsigned short queue[kNbrThreads / 32][32 * (kNbrScan + 1)];
     __shared__ double rshift[54][3];
-    __shared__ int nst;
     const int cell = blockIdx.x;
-    const int hs = cstart[cell], he = cend[cell];
-    if (he <= hs) return;  // empty cell: the whole block leaves
+    // this block's share of the cell's sites (gridDim.y blocks per cell)
+    const int c_lo = cstart[cell], c_hi = cend[cell], share = (c_hi - c_lo + (int)gridDim.y - 1) / (int)gridDim.y;
+    const int hs = c_lo + (int)blockIdx.y * share, he = min(c_hi, hs + share);
+    if (he <= hs) return;  // nothing to do: the whole block leaves
     const int c2 = cell % cg.nc[2], c1 = (cell / cg.nc[2]) % cg.nc[1], c0 = cell / (cg.nc[2] * cg.nc[1]);
     const int cc[3] = {c0, c1, c2};
     double corner[3];
@@ -380,15 +388,12 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_cells(
                 if ((int)threadIdx.x >= o) incl += v;
             }
             if (k < total) rpre[k] = carry + incl - len;
-            if (k == total - 1) {
-                rpre[total] = carry + incl;
-                nst = total;
-            }
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
+        for (int k = total + (int)threadIdx.x; k < 64; k += 32) rpre[k] = carry;
     }
     __syncthreads();
-    const int M = rpre[nst];
+    const int M = rpre[63];
     // position in the box (periodic) relative to the home cell's corner;
     // a general cell wraps the fractional coordinates
     auto rel3 = [&](const double4& x, double (&o)[3]) {
@@ -431,74 +436,107 @@ __global__ void __launch_bounds__(kNbrThreads) k_neighbors_cells(
         for (int m0 = 0; m0 < M; m0 += kNbrChunk) {
             const int mn = min(kNbrChunk, M - m0);
             __syncthreads();  // the previous chunk is consumed and hcnt is initialised
-            // stage the chunk one stencil cell at a time (cells overlapping it)
-            for (int k = 0; k < nst; k++) {
-                const int f0 = max(rpre[k], m0), f1 = min(rpre[k + 1], m0 + mn);
-                for (int f = f0 + threadIdx.x; f < f1; f += blockDim.x) {
-                    const int p = rstart[k] + (f - rpre[k]);
-                    double c3[3];
-                    rel3(spos[p], c3);
-                    const int t = f - m0;
-                    cpos[t] = make_float4((float)(c3[0] + rshift[k][0]), (float)(c3[1] + rshift[k][1]),
-                                          (float)(c3[2] + rshift[k][2]), 0.f);
-                    csrt[t] = p;
-                    cid[t] = sids[p];
+            // stage the chunk, a candidate per thread: its stencil cell by
+            // bisection of the cells' first candidates (the loads of all
+            // cells in flight together); past the end, a point out of reach
+            for (int t = threadIdx.x; t < ((mn + 31) & ~31); t += blockDim.x) {
+                if (t >= mn) {
+                    cpos[t] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+                    continue;
                 }
+                const int f = m0 + t;
+                int k = 0;
+#pragma unroll
+                for (int o = 32; o > 0; o >>= 1)
+                    if (rpre[k + o] <= f) k += o;
+                const int p = rstart[k] + (f - rpre[k]);
+                double c3[3];
+                rel3(spos[p], c3);
+                cpos[t] = make_float4((float)(c3[0] + rshift[k][0]), (float)(c3[1] + rshift[k][1]),
+                                      (float)(c3[2] + rshift[k][2]), 0.f);
+                csrt[t] = p;
+                cid[t] = sids[p];
             }
             __syncthreads();
+            unsigned short* q = queue[warp];
             for (int hh = warp; hh < hn; hh += nwarp) {
                 const int ph = h0 + hh;
                 const int i = hid[hh];
                 const float4 hp = hpos[hh];
                 const float hx = hp.x, hy = hp.y, hz = hp.z;
-                const int x0 = hx0[hh], x1 = hx1[hh];
+                const int x0 = hx0[hh], nx = hx1[hh] - x0;
                 const int2 xr = hxr[hh];  // index range of i's scaled partners
-                const int limit = cap - (x1 - x0);  // the row's tail holds the scaled partners
-                // the first kExcl scaled partners in registers, the rest read when needed
-                constexpr int kExcl = 8;
-                int ex[kExcl];
-#pragma unroll
-                for (int q = 0; q < kExcl; q++) ex[q] = x0 + q < x1 ? xidx[x0 + q] : -1;
+                const int limit = cap - nx;  // the row's tail holds the scaled partners
+                const int ex = lane < nx ? xidx[x0 + lane] : -1;  // the first 32 scaled partners, a lane each
                 int* row = nbr + (size_t)i * cap;
+                int* rowc = cnb + (size_t)i * cap;
                 int cnt = hcnt[hh];
-                for (int b = 0; b < mn; b += 32) {
-                    const int t = b + lane;
+                // the first `len` (up to 32) queued candidates: those that are partners go to the row
+                auto decide = [&](int len) {
                     bool hit = false;
-                    int j = -1;
-                    if (t < mn) {
+                    int j = -1, p = 0;
+                    if (lane < len) {
+                        const int t = q[lane];
+                        j = cid[t];
+                        p = csrt[t];
                         const float4 c = cpos[t];
                         const float dx = c.x - hx, dy = c.y - hy, dz = c.z - hz;
-                        const float r2 = dx * dx + dy * dy + dz * dz;
-                        if (r2 <= hi2) {
-                            j = cid[t];
-                            hit = j != i;
-                            // near the cutoff the FP64 minimum image decides; in a
-                            // general cell it decides every pair, so the pair set
-                            // is that of the cell's image(), as in k_neighbors
-                            if (hit && (r2 > lo2 || GENERAL || CENTRED)) {
-                                const double4 xi = spos[ph];
-                                const double4 pj = spos[csrt[t]];
-                                const V3<double> r = min_image<double, GENERAL || CENTRED>(
-                                    v3<double>(pj.x - xi.x, pj.y - xi.y, pj.z - xi.z), bx);
-                                hit = dot(r, r) <= cut2;
-                            }
-                            if (hit && j >= xr.x && j <= xr.y) {  // only then can j be a scaled partner
-#pragma unroll
-                                for (int q = 0; q < kExcl; q++) hit &= (ex[q] != j);
-                                for (int q = x0 + kExcl; q < x1; q++) hit &= (xidx[q] != j);
-                            }
+                        hit = j != i;
+                        // near the cutoff the FP64 minimum image decides; in a
+                        // general cell it decides every pair, so the pair set
+                        // is that of the cell's image(), as in k_neighbors
+                        if (hit && (GENERAL || CENTRED || dx * dx + dy * dy + dz * dz > lo2)) {
+                            const double4 xi = spos[ph];
+                            const double4 pj = spos[p];
+                            const V3<double> r = min_image<double, GENERAL || CENTRED>(
+                                v3<double>(pj.x - xi.x, pj.y - xi.y, pj.z - xi.z), bx);
+                            hit = dot(r, r) <= cut2;
                         }
                     }
+                    if (__any_sync(0xffffffffu, hit && j >= xr.x && j <= xr.y))  // only then can j be a scaled partner
+                        for (int e = 0; e < nx; e++)
+                            hit &= (e < 32 ? __shfl_sync(0xffffffffu, ex, e) : xidx[x0 + e]) != j;
                     const unsigned m = __ballot_sync(0xffffffffu, hit);
                     if (hit) {
                         const int pos = cnt + __popc(m & below);
                         if (pos < limit) {
                             row[pos] = j;
-                            cnb[(size_t)i * cap + pos] = csrt[t];  // the partner's position in cell order
+                            rowc[pos] = p;  // the partner's position in cell order
                         }
                     }
                     cnt += __popc(m);
+                };
+                int qn = 0;
+                for (int b = 0; b < mn; b += 32 * kNbrScan) {
+                    bool near[kNbrScan];
+#pragma unroll
+                    for (int u = 0; u < kNbrScan; u++) {
+                        const int t = b + 32 * u + lane;
+                        const float4 c = cpos[min(t, kNbrChunk - 1)];
+                        const float dx = c.x - hx, dy = c.y - hy, dz = c.z - hz;
+                        near[u] = b + 32 * u < mn && dx * dx + dy * dy + dz * dz <= hi2;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kNbrScan; u++) {
+                        const unsigned m = __ballot_sync(0xffffffffu, near[u]);
+                        if (near[u]) q[qn + __popc(m & below)] = (unsigned short)(b + 32 * u + lane);
+                        qn += __popc(m);
+                    }
+                    __syncwarp();
+                    while (qn >= 32) {
+                        decide(32);
+                        qn -= 32;
+                        unsigned short keep[kNbrScan];  // the rest of the queue moves to its front
+#pragma unroll
+                        for (int u = 0; u < kNbrScan; u++) keep[u] = q[32 * (u + 1) + lane];
+                        __syncwarp();
+#pragma unroll
+                        for (int u = 0; u < kNbrScan; u++) q[32 * u + lane] = keep[u];
+                        __syncwarp();
+                    }
                 }
+                if (qn) decide(qn);
+                __syncwarp();
                 if (lane == 0) hcnt[hh] = cnt;
             }
         }
