@@ -31,7 +31,7 @@ using namespace amg;
 namespace {
 
 constexpr int kOrder = 5;        // B-spline order compiled in (pme.h bseorder default)
-constexpr int kGatherLanes = 8;  // lanes per site in the PME derivative gathers
+constexpr int kGatherLanes = 4;  // lanes per site in the PME gathers (8: within 3% either way up to 12,288 sites, slower above)
 constexpr int kThreads = 128;
 constexpr int kRbChunks = 8;  // pieces of the gradient read-back
 // FP64 accumulators (eacc): em real 0, einter 1, em reciprocal 2, net charge
@@ -85,6 +85,7 @@ struct Pme {
     typename CufftTypes<R>::C* cgrid = nullptr;  // [2][K1 K2 (K3/2+1)]
     R* infl = nullptr;                       // [K1 K2 (K3/2+1)]
     R* theta = nullptr;                      // [n][3][4][P]
+    R* rec = nullptr;                        // [n][kRecWords] field records
     int* k0 = nullptr;                       // [n][3]
     cufftHandle f1 = 0, i1 = 0, zplan = 0;
     // dipole grids: d + i p interleaved, transformed in place
@@ -405,6 +406,7 @@ void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
         dalloc(ctx, pm.infl, pm.Gc);
         dalloc(ctx, pm.theta, (size_t)ctx->n * 3 * 4 * kOrder);
         dalloc(ctx, pm.k0, (size_t)ctx->n * 3);
+        dalloc(ctx, pm.rec, (size_t)ctx->n * kRecWords);
         int dims[3] = {K1, K2, K3};
         CKFFT(cufftPlanMany(&pm.f1, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CufftTypes<R>::r2c, 1));
         CKFFT(cufftPlanMany(&pm.i1, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CufftTypes<R>::c2r, 1));
@@ -470,7 +472,7 @@ void pme_destroy(Pme<R>& pm) {
     for (int k = 0; k < 3; k++)
         if (*hs[k]) { cufftDestroy(*hs[k]); *hs[k] = 0; }
     dfree(pm.zg); dfree(pm.zq); dfree(pm.Gfull);
-    dfree(pm.grid); dfree(pm.phig); dfree(pm.cgrid); dfree(pm.infl); dfree(pm.theta); dfree(pm.k0);
+    dfree(pm.grid); dfree(pm.phig); dfree(pm.cgrid); dfree(pm.infl); dfree(pm.theta); dfree(pm.k0); dfree(pm.rec);
     pm.ready = false;
 }
 
@@ -830,20 +832,15 @@ void pme_stencils(amg_ctx* ctx, cudaStream_t s, bool with_fp64 = false) {
     constexpr int BS = 64;
     const unsigned blocks = (unsigned)((ctx->n + BS - 1) / BS);
     const int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
-    if constexpr (sizeof(R) == 8) {
-        Pme<double>& pd = pme_of<double>(ctx);
-        k_bspline_rows<kOrder, BS, true, false><<<blocks, BS, 0, s>>>(ctx->n, ctx->xyz, ctx->bx, ctx->frac, K, pd.theta,
-                                                                      pd.k0, nullptr, nullptr);
-    } else if (with_fp64) {
-        Pme<double>& pd = pme_of<double>(ctx);
-        Pme<float>& pf = pme_of<float>(ctx);
-        k_bspline_rows<kOrder, BS, true, true><<<blocks, BS, 0, s>>>(ctx->n, ctx->xyz, ctx->bx, ctx->frac, K, pd.theta,
-                                                                     pd.k0, pf.theta, pf.k0);
-    } else {
-        Pme<float>& pf = pme_of<float>(ctx);
-        k_bspline_rows<kOrder, BS, false, true><<<blocks, BS, 0, s>>>(ctx->n, ctx->xyz, ctx->bx, ctx->frac, K, nullptr,
-                                                                      nullptr, pf.theta, pf.k0);
-    }
+    Pme<double>& pd = pme_of<double>(ctx);
+    Pme<float>& pf = pme_of<float>(ctx);
+    auto launch = [&](auto kern) {
+        kern<<<blocks, BS, 0, s>>>(ctx->n, ctx->xyz, ctx->bx, ctx->frac, K, pd.theta, pd.k0, pd.rec, pf.theta, pf.k0,
+                                   pf.rec);
+    };
+    if constexpr (sizeof(R) == 8) launch(k_bspline_rows<kOrder, BS, true, false>);
+    else if (with_fp64) launch(k_bspline_rows<kOrder, BS, true, true>);
+    else launch(k_bspline_rows<kOrder, BS, false, true>);
     KCHECK();
 }
 
@@ -888,9 +885,8 @@ template <class R>
 void spread_dipoles(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp) {
     Pme<R>& pm = pme_of<R>(ctx);
     int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
-    k_spread_dipoles<R, kOrder><<<spread_blocks<R>(ctx->n), 128, 0, s>>>(ctx->n, ctx->sids, vd, vp, pm.theta, pm.k0,
-                                                                          K, ctx->frac,
-                                                        pm.zg);
+    k_spread_dipoles<R, kOrder><<<spread_blocks<R>(ctx->n), 128, 0, s>>>(ctx->n, ctx->sids, vd, vp, pm.rec, K,
+                                                                          ctx->frac, pm.zg);
     KCHECK();
 }
 
@@ -1077,10 +1073,9 @@ void matvec_stored(amg_ctx* ctx, cudaStream_t s, const R4<R>* v4, const double* 
         pme_dipole_grids<R>(ctx, s, vd, vp, spread, nullptr, true, clear);
         if (!apart) join_side(ctx, s);
         int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
-        constexpr int G = 8;  // lanes per site
+        constexpr int G = kGatherLanes;
         const unsigned blocks = (unsigned)std::min<size_t>(nblk((size_t)n * G), (size_t)ctx->num_sms * 8);
-        k_gather_field<R, kOrder, G><<<blocks, kThreads, 0, s>>>(n, pm.zq, pm.theta, pm.k0, K, ctx->frac, vd,
-                                                                 vp, apart ? nullptr : ctx->Fd,
+        k_gather_field<R, kOrder, G><<<blocks, kThreads, 0, s>>>(n, pm.zq, pm.rec, K, ctx->frac, vd, vp, apart ? nullptr : ctx->Fd,
                                                                  apart ? nullptr : ctx->Fp, self_coef(ctx), ctx->pol,
                                                                  Ad, Ap, vAv);
         KCHECK();
@@ -1132,8 +1127,8 @@ void direction(amg_ctx* ctx, cudaStream_t s) {
     if (ctx->ewald && !split_spread(ctx)) {
         Pme<R>& pm = pme_of<R>(ctx);
         const int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
-        k_pcg_dir_spread<R, kOrder><<<spread_blocks<R>(n), 128, 0, s>>>(n, ctx->zd, ctx->zp, ctx->pd, ctx->pp, ctx->scal, A.p4, pm.theta,
-                                                       pm.k0, K, ctx->frac, pm.zg, ctx->rank);
+        k_pcg_dir_spread<R, kOrder><<<spread_blocks<R>(n), 128, 0, s>>>(n, ctx->zd, ctx->zp, ctx->pd, ctx->pp, ctx->scal, A.p4, pm.rec, K,
+                                                       ctx->frac, pm.zg, ctx->rank);
     } else {
         k_pcg_dir<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->zd, ctx->zp, ctx->pd, ctx->pp, ctx->scal, A.p4, ctx->rank);
     }

@@ -221,8 +221,8 @@ template <class R, int P>
 __global__ void __launch_bounds__(128) k_pcg_dir_spread(int n, const double* __restrict__ zd,
                                                         const double* __restrict__ zp, double* __restrict__ pd,
                                                         double* __restrict__ pp, const double* __restrict__ scal,
-                                                        R4<R>* __restrict__ p4, const R* __restrict__ theta,
-                                                        const int* __restrict__ k0, int3 K, Frac F,
+                                                        R4<R>* __restrict__ p4, const R* __restrict__ rec, int3 K,
+                                                        Frac F,
                                                         typename Cplx<R>::type* __restrict__ zg,
                                                         const int* __restrict__ rank) {
     constexpr int SPB = sizeof(R) == 8 ? 1 : kLineSites;  // sites per block
@@ -248,11 +248,11 @@ __global__ void __launch_bounds__(128) k_pcg_dir_spread(int n, const double* __r
     }
     if constexpr (SPB == 1) {
         if (t >= P * P * P || i0 >= n) return;
-        spread_site_point<R, P>(i0, t, pv[0], pv[0] + 3, theta, k0, K, F, zg);
+        spread_site_point<R, P>(i0, t, pv[0], pv[0] + 3, rec, K, F, zg);
     } else {
         const int s = t / (P * P), i = i0 + s;
         if (t >= SPB * P * P || i >= n) return;
-        spread_site_line<R, P>(i, t % (P * P), pv[s], pv[s] + 3, theta, k0, K, F, zg);
+        spread_site_line<R, P>(i, t % (P * P), pv[s], pv[s] + 3, rec, K, F, zg);
     }
 }
 

@@ -10,6 +10,9 @@
 // ways as in smooth PME) convolves both sets.
 #pragma once
 #include "kernels.cuh"
+#include "kernels_setup.cuh"
+
+#include <type_traits>
 
 namespace amg {
 
@@ -23,6 +26,18 @@ template <>
 struct Cplx<double> {
     using type = double2;
 };
+
+// two consecutive values, the first at an even place of an aligned array
+__device__ __forceinline__ void load2(const float* __restrict__ p, float& a, float& b) {
+    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+    a = v.x;
+    b = v.y;
+}
+__device__ __forceinline__ void load2(const double* __restrict__ p, double& a, double& b) {
+    const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+    a = v.x;
+    b = v.y;
+}
 
 __device__ __forceinline__ int gidx(int a, int b, int c, int3 K) { return (a * K.y + b) * K.z + c; }
 
@@ -187,20 +202,22 @@ __device__ __forceinline__ void add_line(typename Cplx<R>::type* line, int c0, i
 // vector atomics a line is P dependent pairs of atomics in one thread)
 template <class R, int P>
 __device__ __forceinline__ void spread_site_point(int i, int t, const double* pd, const double* pq,
-                                                  const R* __restrict__ theta, const int* __restrict__ k0, int3 K,
-                                                  const Frac& F, typename Cplx<R>::type* __restrict__ zg) {
+                                                  const R* __restrict__ rec, int3 K, const Frac& F,
+                                                  typename Cplx<R>::type* __restrict__ zg) {
     const int a = t / (P * P), b = (t / P) % P, c = t % P;
-    const R* th = theta + (size_t)i * 3 * 4 * P;
+    const R* th = rec + (size_t)i * kRecWords;
     const R t0 = th[a], t1 = th[P + a];
-    const R u0 = th[4 * P + b], u1 = th[5 * P + b];
-    const R v0 = th[8 * P + c], v1 = th[9 * P + c];
+    const R u0 = th[2 * P + b], u1 = th[3 * P + b];
+    const R v0 = th[4 * P + c], v1 = th[5 * P + c];
     R d0, d1, d2, p0, p1, p2;
     frac_dipole<R>(F, pd[0], pd[1], pd[2], d0, d1, d2);
     frac_dipole<R>(F, pq[0], pq[1], pq[2], p0, p1, p2);
     const R w100 = t1 * u0 * v0, w010 = t0 * u1 * v0, w001 = t0 * u0 * v1;
-    int ga = k0[3 * i] + a; if (ga >= K.x) ga -= K.x;
-    int gb = k0[3 * i + 1] + b; if (gb >= K.y) gb -= K.y;
-    int gc = k0[3 * i + 2] + c; if (gc >= K.z) gc -= K.z;
+    int ga, gb, gc;
+    load_start<P>(th, ga, gb, gc);
+    ga += a; if (ga >= K.x) ga -= K.x;
+    gb += b; if (gb >= K.y) gb -= K.y;
+    gc += c; if (gc >= K.z) gc -= K.z;
     add_cplx<R>(zg + gidx(ga, gb, gc, K), d0 * w100 + d1 * w010 + d2 * w001, p0 * w100 + p1 * w010 + p2 * w001);
 }
 
@@ -208,13 +225,18 @@ __device__ __forceinline__ void spread_site_point(int i, int t, const double* pd
 // (p set), converted to fractional dipoles here
 template <class R, int P>
 __device__ __forceinline__ void spread_site_line(int i, int l, const double* pd, const double* pq,
-                                                 const R* __restrict__ theta, const int* __restrict__ k0, int3 K,
-                                                 const Frac& F, typename Cplx<R>::type* __restrict__ zg) {
+                                                 const R* __restrict__ rec, int3 K, const Frac& F,
+                                                 typename Cplx<R>::type* __restrict__ zg) {
     static_assert(P % 2 == 1, "the pairing of line points assumes an odd order");
     const int a = l / P, b = l % P;
-    const R* th = theta + (size_t)i * 3 * 4 * P;
+    const R* th = rec + (size_t)i * kRecWords;
     const R t0 = th[a], t1 = th[P + a];
-    const R u0 = th[4 * P + b], u1 = th[5 * P + b];
+    const R u0 = th[2 * P + b], u1 = th[3 * P + b];
+    R z[2 * P];  // z weights, then their first derivatives
+#pragma unroll
+    for (int c = 0; c < 2 * P; c += 2) load2(th + 4 * P + c, z[c], z[c + 1]);
+    int ga, gb, gc;
+    load_start<P>(th, ga, gb, gc);
     R d0, d1, d2, p0, p1, p2;
     frac_dipole<R>(F, pd[0], pd[1], pd[2], d0, d1, d2);
     frac_dipole<R>(F, pq[0], pq[1], pq[2], p0, p1, p2);
@@ -224,20 +246,18 @@ __device__ __forceinline__ void spread_site_line(int i, int l, const double* pd,
     R vx[P], vy[P];
 #pragma unroll
     for (int c = 0; c < P; c++) {
-        const R v0 = th[8 * P + c], v1 = th[9 * P + c];
-        vx[c] = ad * v0 + bd * v1;
-        vy[c] = ap * v0 + bp * v1;
+        vx[c] = ad * z[c] + bd * z[P + c];
+        vy[c] = ap * z[c] + bp * z[P + c];
     }
-    int ga = k0[3 * i] + a; if (ga >= K.x) ga -= K.x;
-    int gb = k0[3 * i + 1] + b; if (gb >= K.y) gb -= K.y;
-    add_line<R, P>(zg + ((size_t)ga * K.y + gb) * K.z, k0[3 * i + 2], K.z, vx, vy);
+    ga += a; if (ga >= K.x) ga -= K.x;
+    gb += b; if (gb >= K.y) gb -= K.y;
+    add_line<R, P>(zg + ((size_t)ga * K.y + gb) * K.z, gc, K.z, vx, vy);
 }
 
 template <class R, int P>
 __global__ void __launch_bounds__(128) k_spread_dipoles(int n, const int* __restrict__ order,
                                                         const double* __restrict__ ud,
-                                                        const double* __restrict__ up,
-                                                        const R* __restrict__ theta, const int* __restrict__ k0,
+                                                        const double* __restrict__ up, const R* __restrict__ rec,
                                                         int3 K, Frac F,
                                                         typename Cplx<R>::type* __restrict__ zg) {
     static_assert(kLineSites * P * P <= 128, "lines of a block");
@@ -245,12 +265,12 @@ __global__ void __launch_bounds__(128) k_spread_dipoles(int n, const int* __rest
     if constexpr (sizeof(R) == 8) {  // FP64: one site per block, one stencil point per thread
         if (t >= P * P * P) return;
         const int i = order[blockIdx.x];
-        spread_site_point<R, P>(i, t, ud + 3 * i, up + 3 * i, theta, k0, K, F, zg);
+        spread_site_point<R, P>(i, t, ud + 3 * i, up + 3 * i, rec, K, F, zg);
     } else {
         const int g = blockIdx.x * kLineSites + t / (P * P);
         if (t >= kLineSites * P * P || g >= n) return;
         const int i = order[g];
-        spread_site_line<R, P>(i, t % (P * P), ud + 3 * i, up + 3 * i, theta, k0, K, F, zg);
+        spread_site_line<R, P>(i, t % (P * P), ud + 3 * i, up + 3 * i, rec, K, F, zg);
     }
 }
 
@@ -260,57 +280,88 @@ inline unsigned spread_blocks(int n) {
     return sizeof(R) == 8 ? (unsigned)n : (unsigned)((n + kLineSites - 1) / kLineSites);
 }
 
-// The P grid values z = c0 .. c0+P-1 (periodic in Kz) of one z-line of the
-// complex dipole grid.  With the line's z-range inside the grid and Kz even,
-// from three aligned loads of two values each (16 bytes in FP32, 32 in FP64)
-// and a select by the parity of c0, instead of one load per value: 6 values
-// cover any 5 consecutive ones; else value by value.  (Two 256-bit FP32
-// loads of 8 values were slower: 64 bytes through L1 for 40 used.)  The grid
-// is read-only in the gathers.
-template <int P>
-__device__ __forceinline__ void load_line(const float2* __restrict__ line, int c0, int Kz, float2 (&q)[P]) {
-    static_assert(P <= 5, "a line of at most 5 values fits 6 loaded ones");
-    const int zb = c0 & ~1, o = c0 & 1;
-    if ((Kz & 1) == 0 && zb + 6 <= Kz) {
-        float4 w[3];
+// The z-lines of a site's stencil are read by 4 consecutive lanes, so that a
+// load instruction touches one run of memory per line (8 to 10 cache lines for
+// the 8 lines of a warp) instead of one cache line per lane, which made the
+// L1 pipe the bound of the gathers; now latency is (98,304 sites, 108^3:
+// k_gather_field 35.6 -> 29.2 us, k_gather<20> of both sets 76 -> 48, of the
+// permanent grid 42 -> 33; FP64, 24,044 sites: k_gather_field 23.5 -> 16.1).  Each lane holds two points of every line and their
+// z weights.  K3 even: lane p takes the aligned pair of points zb + 2p, zb +
+// 2p + 1 (zb = c0 rounded down to even; a pair never straddles the wrap) in
+// one vector load; 3 pairs hold any 5 consecutive points, and lane 3 reads
+// lane 2's pair with zero weights.  K3 odd: lane p takes the points c0 + p
+// and (lane 0) c0 + 4, value by value.
+constexpr int kLineLanes = 4;
+
+template <class R, int P, int ND>
+struct LineLane {
+    int z0, z1;       // grid indices of the lane's two points
+    R w0[ND], w1[ND]; // their weights, by derivative order
+    __device__ __forceinline__ LineLane(int p, int c0, int Kz, const R* __restrict__ t3) {
+        static_assert(P == 5, "two points per lane hold a line of 5");
+        int a, b;  // the points' places in the stencil
+        if ((Kz & 1) == 0) {
+            const int zb = c0 & ~1;
+            z0 = zb + 2 * min(p, 2);
+            if (z0 >= Kz) z0 -= Kz;
+            z1 = z0 + 1;
+            a = zb + 2 * p - c0;
+            b = a + 1;
+        } else {
+            a = p;
+            b = p == 0 ? 4 : P;
+            z0 = c0 + p;
+            z1 = c0 + 4;
+            if (z0 >= Kz) z0 -= Kz;
+            if (z1 >= Kz) z1 -= Kz;
+        }
+        const bool oka = a >= 0 && a < P, okb = b < P;
 #pragma unroll
-        for (int h = 0; h < 3; h++) w[h] = __ldg(reinterpret_cast<const float4*>(line + zb) + h);
-        const float2 v[6] = {make_float2(w[0].x, w[0].y), make_float2(w[0].z, w[0].w), make_float2(w[1].x, w[1].y),
-                             make_float2(w[1].z, w[1].w), make_float2(w[2].x, w[2].y), make_float2(w[2].z, w[2].w)};
-#pragma unroll
-        for (int c = 0; c < P; c++) q[c] = o ? v[c + 1] : v[c];
-        return;
+        for (int d = 0; d < ND; d++) {
+            w0[d] = oka ? t3[d * P + a] : R(0);
+            w1[d] = okb ? t3[d * P + b] : R(0);
+        }
     }
-#pragma unroll
-    for (int c = 0; c < P; c++) {
-        int gc = c0 + c;
-        if (gc >= Kz) gc -= Kz;
-        q[c] = line[gc];
+};
+
+// the two points of a line for this lane: NS = 2, both dipole sets (d0, p0,
+// d1, p1); NS = 1, a real grid (q0, q1).  The grids are read-only in the gathers.
+__device__ __forceinline__ void line_points(const float2* __restrict__ line, int z0, int z1, bool even, float (&q)[4]) {
+    if (even) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(line + z0));
+        q[0] = v.x; q[1] = v.y; q[2] = v.z; q[3] = v.w;
+    } else {
+        const float2 a = __ldg(line + z0), b = __ldg(line + z1);
+        q[0] = a.x; q[1] = a.y; q[2] = b.x; q[3] = b.y;
     }
 }
-template <int P>
-__device__ __forceinline__ void load_line(const double2* __restrict__ line, int c0, int Kz, double2 (&q)[P]) {
-    static_assert(P <= 5, "a line of at most 5 values fits 6 loaded ones");
-    const int zb = c0 & ~1, o = c0 & 1;
-    if ((Kz & 1) == 0 && zb + 6 <= Kz) {
-        double w[12];
-#pragma unroll
-        for (int h = 0; h < 3; h++)
-            asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-                : "=d"(w[4 * h]), "=d"(w[4 * h + 1]), "=d"(w[4 * h + 2]), "=d"(w[4 * h + 3])
-                : "l"(line + zb + 2 * h));
-#pragma unroll
-        for (int c = 0; c < P; c++) {
-            q[c].x = o ? w[2 * c + 2] : w[2 * c];
-            q[c].y = o ? w[2 * c + 3] : w[2 * c + 1];
-        }
-        return;
+__device__ __forceinline__ void line_points(const double2* __restrict__ line, int z0, int z1, bool even,
+                                            double (&q)[4]) {
+    if (even) {
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(q[0]), "=d"(q[1]), "=d"(q[2]), "=d"(q[3]) : "l"(line + z0));
+    } else {
+        const double2 a = __ldg(line + z0), b = __ldg(line + z1);
+        q[0] = a.x; q[1] = a.y; q[2] = b.x; q[3] = b.y;
     }
-#pragma unroll
-    for (int c = 0; c < P; c++) {
-        int gc = c0 + c;
-        if (gc >= Kz) gc -= Kz;
-        q[c] = line[gc];
+}
+__device__ __forceinline__ void line_points(const float* __restrict__ line, int z0, int z1, bool even, float (&q)[2]) {
+    if (even) {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(line + z0));
+        q[0] = v.x; q[1] = v.y;
+    } else {
+        q[0] = __ldg(line + z0);
+        q[1] = __ldg(line + z1);
+    }
+}
+__device__ __forceinline__ void line_points(const double* __restrict__ line, int z0, int z1, bool even,
+                                            double (&q)[2]) {
+    if (even) {
+        const double2 v = __ldg(reinterpret_cast<const double2*>(line + z0));
+        q[0] = v.x; q[1] = v.y;
+    } else {
+        q[0] = __ldg(line + z0);
+        q[1] = __ldg(line + z1);
     }
 }
 
@@ -319,74 +370,119 @@ __device__ __forceinline__ void load_line(const double2* __restrict__ line, int 
 // matvec assembly:
 //   A v = v/alpha - (F_real + F_recip + selfc v),  F_recip = -grad phi
 // and, when vAv is given, the PCG dot products v.Av of both sets added to
-// vAv[0], vAv[1].  G consecutive lanes per site; each lane takes whole
-// z-lines (a, b) of the P^3 stencil (P grid values per line), the per-lane
-// sums are combined with shuffles and lanes 0..5 write the six components.
+// vAv[0], vAv[1].  kLineLanes lanes per z-line (LineLane), G lanes per site:
+// with G = 8 the two halves share the x planes of the stencil.  Each lane
+// contracts its points of a plane's lines with the y weights, the planes with
+// the x weights and only the result with the z weights; the lanes' sums are
+// combined with shuffles and the lanes write the six components, whose
+// operands were requested first (35 -> 29 us: the kernel waits on memory).
 // Blocks stride over the sites, so each block adds its dot products once.
 // With Fd, Fp null the real-space field is left out (A v without -F_real,
 // and its dot products): the real-space kernel then runs beside this one and
 // adds its own share (k_tu_stored with vAv), and k_pcg_update subtracts F.
 template <class R, int P, int G>
 __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx<R>::type* __restrict__ zg,
-                                                      const R* __restrict__ theta, const int* __restrict__ k0,
-                                                      int3 K, Frac F,
+                                                      const R* __restrict__ rec, int3 K, Frac F,
                                                       const double* __restrict__ vd, const double* __restrict__ vp,
                                                       const double* __restrict__ Fd, const double* __restrict__ Fp,
                                                       double selfc, const double* __restrict__ pol,
                                                       double* __restrict__ Ad, double* __restrict__ Ap,
                                                       double* __restrict__ vAv) {
-    const int lane = threadIdx.x % G, per_block = blockDim.x / G;
+    constexpr int S = G / kLineLanes, NA = (P + S - 1) / S;  // sub-groups of a site, x planes of each
+    const int lane = threadIdx.x % G, per_block = blockDim.x / G, sub = lane / kLineLanes;
+    const bool even = (K.z & 1) == 0;
     double dotd = 0, dotp = 0;  // v.Av of this thread's components
     for (int g0 = blockIdx.x * per_block; g0 < n; g0 += gridDim.x * per_block) {
         const int g = g0 + threadIdx.x / G;
         const int i = min(g, n - 1);
-        const R* th = theta + (size_t)i * 3 * 4 * P;
-        const int a0 = k0[3 * i], b0 = k0[3 * i + 1], c0 = k0[3 * i + 2];
-        R v0[P], v1[P];
-#pragma unroll
-        for (int c = 0; c < P; c++) {
-            v0[c] = th[8 * P + c];
-            v1[c] = th[9 * P + c];
+        const R* th = rec + (size_t)i * kRecWords;
+        int a0, b0, c0;
+        load_start<P>(th, a0, b0, c0);
+        // what the lane needs at the end, on its way while the grid is read:
+        // of each pair of lanes the first takes x and z, the second y
+        const bool pset = lane & 2;
+        const double* vv = pset ? vp : vd;
+        const double* FF = pset ? Fp : Fd;
+        const double alpha = pol[i];
+        double ve[2], fe[2] = {0, 0};
+        const int q0 = 3 * i + (lane & 1), q1 = 3 * i + 2;
+        ve[0] = vv[q0];
+        ve[1] = vv[q1];
+        if (FF) {
+            fe[0] = FF[q0];
+            fe[1] = FF[q1];
         }
-        R f[6] = {0, 0, 0, 0, 0, 0};
-        for (int l = lane; l < P * P; l += G) {
-            const int a = l / P, b = l - (l / P) * P;
-            int ga = a0 + a; if (ga >= K.x) ga -= K.x;
+        const LineLane<R, P, 2> L(lane % kLineLanes, c0, K.z, th + 4 * P);
+        R u[2 * P];   // y weights, then their first derivatives
+        int row[P];   // offsets of the stencil's rows y
+#pragma unroll
+        for (int b = 0; b < P; b++) {
+            load2(th + 2 * P + 2 * b, u[2 * b], u[2 * b + 1]);
             int gb = b0 + b; if (gb >= K.y) gb -= K.y;
-            const typename Cplx<R>::type* line = zg + ((size_t)ga * K.y + gb) * K.z;
-            typename Cplx<R>::type qv[P];
-            load_line<P>(line, c0, K.z, qv);
-            R sd0 = 0, sd1 = 0, sp0 = 0, sp1 = 0;
-#pragma unroll
-            for (int c = 0; c < P; c++) {
-                const R qd = qv[c].x, qp = qv[c].y;
-                sd0 += v0[c] * qd; sd1 += v1[c] * qd;
-                sp0 += v0[c] * qp; sp1 += v1[c] * qp;
-            }
-            const R t0 = th[a], t1 = th[P + a], u0 = th[4 * P + b], u1 = th[5 * P + b];
-            const R w100 = t1 * u0, w010 = t0 * u1, w001 = t0 * u0;
-            f[0] += w100 * sd0; f[1] += w010 * sd0; f[2] += w001 * sd1;
-            f[3] += w100 * sp0; f[4] += w010 * sp0; f[5] += w001 * sp1;
+            row[b] = gb * K.z;
         }
-        double sum[6];
+        // sums over x and y of the lane's four values (d, p at z0, d, p at
+        // z1) with the weights' orders (1, 0), (0, 1), (0, 0)
+        R s10[4] = {0, 0, 0, 0}, s01[4] = {0, 0, 0, 0}, s00[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int k = 0; k < 6; k++) sum[k] = group_sum<G>((double)f[k]);
-        if (g < n && lane < 6) {
-            const int t = lane, c = t % 3;
-            const bool dset = t < 3;
-            // d phi / dx_c from the grid-unit first derivatives of this set
-            const double s0 = dset ? sum[0] : sum[3], s1 = dset ? sum[1] : sum[4], s2 = dset ? sum[2] : sum[5];
-            const double dphi = F.general ? F.m[c][0] * s0 + F.m[c][1] * s1 + F.m[c][2] * s2
-                                          : F.m[c][c] * (c == 0 ? s0 : c == 1 ? s1 : s2);
-            const double* vv = dset ? vd : vp;
-            const double* FF = dset ? Fd : Fp;
-            double* AA = dset ? Ad : Ap;
-            const double alpha = pol[i];
-            const double field = (FF ? FF[3 * i + c] : 0.0) - dphi + selfc * vv[3 * i + c];
-            const double av = alpha > 0 ? vv[3 * i + c] / alpha - field : 0.0;
-            AA[3 * i + c] = av;
-            if (dset) dotd += vv[3 * i + c] * av;
-            else dotp += vv[3 * i + c] * av;
+        for (int aa = 0; aa < NA; aa++) {
+            const int a = sub * NA + aa;
+            if (S > 1 && a >= P) break;
+            int ga = a0 + a; if (ga >= K.x) ga -= K.x;
+            const typename Cplx<R>::type* plane = zg + (size_t)ga * K.y * K.z;
+            R q[P][4];
+#pragma unroll
+            for (int b = 0; b < P; b++) line_points(plane + row[b], L.z0, L.z1, even, q[b]);
+            const R t0 = th[a], t1 = th[P + a];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                R y0 = 0, y1 = 0;
+#pragma unroll
+                for (int b = 0; b < P; b++) {
+                    y0 += u[b] * q[b][v];
+                    y1 += u[P + b] * q[b][v];
+                }
+                s10[v] += t1 * y0;
+                s01[v] += t0 * y1;
+                s00[v] += t0 * y0;
+            }
+        }
+        // z, then over the lanes: the lower two lanes end with the three sums
+        // of the d set, the upper two with those of the p set
+        double f[6], sum[3];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            f[3 * k] = (double)(L.w0[0] * s10[k] + L.w1[0] * s10[2 + k]);
+            f[3 * k + 1] = (double)(L.w0[0] * s01[k] + L.w1[0] * s01[2 + k]);
+            f[3 * k + 2] = (double)(L.w0[1] * s00[k] + L.w1[1] * s00[2 + k]);
+        }
+        if constexpr (S > 1) {
+#pragma unroll
+            for (int k = 0; k < 6; k++) f[k] += __shfl_xor_sync(0xffffffffu, f[k], kLineLanes);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            sum[k] = (pset ? f[3 + k] : f[k]) + __shfl_xor_sync(0xffffffffu, pset ? f[k] : f[3 + k], 2);
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 1);
+        }
+        if (g < n && sub == 0) {
+            const double ia = 1.0 / alpha;
+            double* AA = pset ? Ap : Ad;
+            double dot = 0;
+            // d phi / dx_c from the grid-unit first derivatives
+            auto finish = [&](double dphi, double v, double ff, int q) {
+                const double av = alpha > 0 ? v * ia - (ff - dphi + selfc * v) : 0.0;
+                AA[q] = av;
+                dot += v * av;
+            };
+            auto deriv = [&](int c) {
+                return F.general ? F.m[c][0] * sum[0] + F.m[c][1] * sum[1] + F.m[c][2] * sum[2] : F.m[c][c] * sum[c];
+            };
+            const double dx = deriv(0), dy = deriv(1);
+            finish((lane & 1) ? dy : dx, ve[0], fe[0], q0);
+            if (!(lane & 1)) finish(deriv(2), ve[1], fe[1], q1);
+            if (pset) dotp += dot;
+            else dotd += dot;
         }
     }
     if (vAv) {
@@ -527,110 +623,86 @@ __global__ void k_convolve(size_t ncomplex, int batch, const R* __restrict__ inf
         for (size_t q = t; q < (size_t)batch * nreal; q += (size_t)gridDim.x * blockDim.x) spread[q] = R(0);
 }
 
-// Gather NC (4, 10 or 20) Cartesian potential derivatives per site:
+// Gather NC (4 or 20) Cartesian potential derivatives per site:
 //   phi_tuv = (K1/L1)^t (K2/L2)^u (K3/L3)^v sum_abc theta1^(t)_a theta2^(u)_b theta3^(v)_c grid
 // from a real grid (NS = 1: grid[g]) or from both parts of the complex
 // dipole grid at once (NS = 2: zg[g].x into phi, zg[g].y into phi + NC n).
-// G consecutive lanes per site; each lane takes whole z-lines (a, b) of the
-// P^3 stencil, contracts the line's P values with the z weights of orders
-// 0..3 and adds them with the x and y weights; the lanes' sums are combined
+// kLineLanes lanes per z-line (LineLane), G lanes per site as in
+// k_gather_field: y, then x, then z contraction, the lanes' sums combined
 // with shuffles.  Output order: 0; x y z; xx yy zz xy xz yz;
 // xxx yyy zzz xxy xxz xyy yyz xzz yzz xyz.
-template <class R, int NC>
-__device__ __forceinline__ void add_derivs(R (&f)[NC], const R (&x)[4], const R (&y)[4], const R (&z)[4]) {
-    f[0] += x[0] * y[0] * z[0];
-    f[1] += x[1] * y[0] * z[0];
-    f[2] += x[0] * y[1] * z[0];
-    f[3] += x[0] * y[0] * z[1];
-    if constexpr (NC >= 10) {
-        f[4] += x[2] * y[0] * z[0];
-        f[5] += x[0] * y[2] * z[0];
-        f[6] += x[0] * y[0] * z[2];
-        f[7] += x[1] * y[1] * z[0];
-        f[8] += x[1] * y[0] * z[1];
-        f[9] += x[0] * y[1] * z[1];
-    }
-    if constexpr (NC >= 20) {
-        f[10] += x[3] * y[0] * z[0];
-        f[11] += x[0] * y[3] * z[0];
-        f[12] += x[0] * y[0] * z[3];
-        f[13] += x[2] * y[1] * z[0];
-        f[14] += x[2] * y[0] * z[1];
-        f[15] += x[1] * y[2] * z[0];
-        f[16] += x[0] * y[2] * z[1];
-        f[17] += x[1] * y[0] * z[2];
-        f[18] += x[0] * y[1] * z[2];
-        f[19] += x[1] * y[1] * z[1];
-    }
-}
+
+// derivative order triples (t, u, v) of the output, in its order
+__device__ constexpr int kDerOut[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0}, {0, 2, 0}, {0, 0, 2},
+                                           {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0},
+                                           {2, 0, 1}, {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}};
 
 template <class R, int P, int NC, int G, int NS>
 __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ gridv, const R* __restrict__ theta,
                                                 const int* __restrict__ k0, int3 K, Frac F,
                                                 double* __restrict__ phi) {
-    constexpr int ND = NC == 4 ? 2 : NC == 10 ? 3 : 4;  // derivative orders per axis
-    using C = typename Cplx<R>::type;
-    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G;
+    static_assert(NC == 4 || NC == 20, "first derivatives, or up to third");
+    constexpr int ND = NC == 4 ? 2 : 4;       // derivative orders per axis
+    constexpr int NV = 2 * NS;                // values of a lane in a line
+    constexpr int S = G / kLineLanes, NA = (P + S - 1) / S;  // sub-groups of a site, x planes of each
+    using E = typename std::conditional<NS == 2, typename Cplx<R>::type, R>::type;
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G, sub = lane / kLineLanes;
     const int i = min(g, n - 1);
+    const bool even = (K.z & 1) == 0;
     const R* t1 = theta + ((size_t)i * 3 + 0) * 4 * P;
     const R* t2 = theta + ((size_t)i * 3 + 1) * 4 * P;
-    const R* t3 = theta + ((size_t)i * 3 + 2) * 4 * P;
     const int a0 = k0[3 * i], b0 = k0[3 * i + 1], c0 = k0[3 * i + 2];
-    int zc[P];
+    const LineLane<R, P, ND> L(lane % kLineLanes, c0, K.z, theta + ((size_t)i * 3 + 2) * 4 * P);
+    R xy[NV][ND][ND];  // sums over x and y with orders (t, u), t + u < ND
 #pragma unroll
-    for (int c = 0; c < P; c++) {
-        int gc = c0 + c;
-        if (gc >= K.z) gc -= K.z;
-        zc[c] = gc;
+    for (int v = 0; v < NV; v++)
+#pragma unroll
+        for (int t = 0; t < ND; t++)
+#pragma unroll
+            for (int u = 0; u + t < ND; u++) xy[v][t][u] = 0;
+    for (int aa = 0; aa < NA; aa++) {
+        const int a = sub * NA + aa;
+        if (S > 1 && a >= P) break;
+        int ga = a0 + a; if (ga >= K.x) ga -= K.x;
+        const E* plane = static_cast<const E*>(gridv) + (size_t)ga * K.y * K.z;
+        R q[P][NV];
+#pragma unroll
+        for (int b = 0; b < P; b++) {
+            int gb = b0 + b; if (gb >= K.y) gb -= K.y;
+            line_points(plane + gb * K.z, L.z0, L.z1, even, q[b]);
+        }
+        R y[NV][ND];
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+#pragma unroll
+            for (int u = 0; u < ND; u++) {
+                y[v][u] = 0;
+#pragma unroll
+                for (int b = 0; b < P; b++) y[v][u] += t2[u * P + b] * q[b][v];
+            }
+#pragma unroll
+        for (int t = 0; t < ND; t++) {
+            const R x = t1[t * P + a];
+#pragma unroll
+            for (int v = 0; v < NV; v++)
+#pragma unroll
+                for (int u = 0; u + t < ND; u++) xy[v][t][u] += x * y[v][u];
+        }
     }
     R f[NS][NC];
 #pragma unroll
     for (int s = 0; s < NS; s++)
 #pragma unroll
-        for (int j = 0; j < NC; j++) f[s][j] = 0;
-    for (int l = lane; l < P * P; l += G) {
-        const int a = l / P, b = l - (l / P) * P;
-        int ga = a0 + a; if (ga >= K.x) ga -= K.x;
-        int gb = b0 + b; if (gb >= K.y) gb -= K.y;
-        const size_t line = ((size_t)ga * K.y + gb) * K.z;
-        R z[NS][4], x[4], y[4];
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-            x[d] = d < ND ? t1[d * P + a] : R(0);
-            y[d] = d < ND ? t2[d * P + b] : R(0);
-#pragma unroll
-            for (int s = 0; s < NS; s++) z[s][d] = 0;
+        for (int j = 0; j < NC; j++) {
+            const int t = kDerOut[j][0], u = kDerOut[j][1], v = kDerOut[j][2];
+            f[s][j] = L.w0[v] * xy[s][t][u] + L.w1[v] * xy[NS + s][t][u];
         }
-        C qv[P];
-        if constexpr (NS == 2) load_line<P>(static_cast<const C*>(gridv) + line, c0, K.z, qv);
-#pragma unroll
-        for (int c = 0; c < P; c++) {
-            R q[NS];
-            if constexpr (NS == 2) {
-                q[0] = qv[c].x;
-                q[NS - 1] = qv[c].y;
-            } else {
-                q[0] = static_cast<const R*>(gridv)[line + zc[c]];
-            }
-#pragma unroll
-            for (int d = 0; d < ND; d++) {
-                const R w = t3[d * P + c];
-#pragma unroll
-                for (int s = 0; s < NS; s++) z[s][d] += w * q[s];
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < NS; s++) add_derivs<R, NC>(f[s], x, y, z[s]);
-    }
     double sum[NS][NC];
 #pragma unroll
     for (int s = 0; s < NS; s++)
 #pragma unroll
         for (int j = 0; j < NC; j++) sum[s][j] = group_sum<G>((double)f[s][j]);
     if (g >= n) return;
-    const int ex[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0}, {0, 2, 0}, {0, 0, 2},
-                           {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0},
-                           {2, 0, 1}, {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}};
     if (F.general) {
 #pragma unroll
         for (int s = 0; s < NS; s++) {
@@ -650,7 +722,8 @@ __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ 
 #pragma unroll
         for (int j = 0; j < NC; j++)
             if (j % G == lane)
-                phi[(size_t)s * NC * n + (size_t)NC * i + j] = sum[s][j] * p0[ex[j][0]] * p1[ex[j][1]] * p2[ex[j][2]];
+                phi[(size_t)s * NC * n + (size_t)NC * i + j] = sum[s][j] * p0[kDerOut[j][0]] * p1[kDerOut[j][1]] *
+                                                             p2[kDerOut[j][2]];
 }
 
 }  // namespace amg

@@ -578,23 +578,55 @@ __device__ __forceinline__ void bspline_weights(double w, R (&th)[4][P]) {
     }
 }
 
+// Field record of a site's stencil: what the dipole kernels (spreading and
+// field gathers, every PCG iteration) need of it in one aligned run of 32
+// words (128 bytes in FP32, one cache line): the weights and first
+// derivatives x0 x1 y0 y1 z0 z1 (P words each), then the three start indices
+// in 64 bits, 21 each.  They read 128 bytes in a few vector loads instead of
+// 192 bytes of the full rows (four orders, 240 bytes) and three indices in
+// single words.
+constexpr int kRecWords = 32;
+
+__device__ __forceinline__ unsigned long long pack_start(int a, int b, int c) {
+    return (unsigned long long)a | (unsigned long long)b << 21 | (unsigned long long)c << 42;
+}
+__device__ __forceinline__ void unpack_start(unsigned long long v, int& a, int& b, int& c) {
+    a = (int)(v & 0x1fffff);
+    b = (int)(v >> 21 & 0x1fffff);
+    c = (int)(v >> 42);
+}
+template <int P>
+__device__ __forceinline__ void load_start(const float* __restrict__ rec, int& a, int& b, int& c) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(rec + 6 * P));
+    unpack_start((unsigned long long)v.y << 32 | v.x, a, b, c);
+}
+template <int P>
+__device__ __forceinline__ void load_start(const double* __restrict__ rec, int& a, int& b, int& c) {
+    unpack_start(__ldg(reinterpret_cast<const unsigned long long*>(rec + 6 * P)), a, b, c);
+}
+
 // B-spline stencils (weights and three derivatives per axis, start indices)
 // of a block of BS sites, computed once in FP64 and
 // written through shared memory, so the block's rows (3 axes x 4 orders x P
 // values per site, consecutive sites adjacent) leave as contiguous runs
 // instead of 60 scattered words per thread; with WD the FP64 stencils, with
 // WF the FP32 copy (the FP32 path rounds the same FP64 values), each with
-// its start indices.
+// its start indices and field records.
 template <int P, int BS, bool WD, bool WF>
 __global__ void __launch_bounds__(BS) k_bspline_rows(int n, const double* __restrict__ xyz, Box bx, Frac F, int3 K,
                                                     double* __restrict__ thd, int* __restrict__ k0d,
-                                                    float* __restrict__ thf, int* __restrict__ k0f) {
+                                                    double* __restrict__ recd, float* __restrict__ thf,
+                                                    int* __restrict__ k0f, float* __restrict__ recf) {
     constexpr int W = 3 * 4 * P;
+    static_assert(P == 5, "a field record holds order-5 stencils");
     __shared__ double sd[BS * W];
+    __shared__ unsigned long long sk[BS];
     const int i0 = blockIdx.x * BS, i = i0 + threadIdx.x;
     if (i < n) {
         const int Ks[3] = {K.x, K.y, K.z};
+        int st[3];
         const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+#pragma unroll
         for (int a = 0; a < 3; a++) {
             double f = F.general ? (x * F.m[0][a] + y * F.m[1][a] + z * F.m[2][a]) / Ks[a]
                                  : (a == 0 ? x : a == 1 ? y : z) * bx.iL[a];
@@ -605,19 +637,34 @@ __global__ void __launch_bounds__(BS) k_bspline_rows(int n, const double* __rest
             bspline_weights<double, P>(u - fl, th);
             int start = (int)fl - P + 1;
             if (start < 0) start += Ks[a];
+            st[a] = start;
             if (WD) k0d[3 * i + a] = start;
             if (WF) k0f[3 * i + a] = start;
             double* o = sd + threadIdx.x * W + a * 4 * P;
             for (int d = 0; d < 4; d++)
                 for (int s = 0; s < P; s++) o[d * P + s] = th[d][s];
         }
+        sk[threadIdx.x] = pack_start(st[0], st[1], st[2]);
     }
     __syncthreads();
-    const int cnt = min(BS, n - i0) * W;
-    for (int t = threadIdx.x; t < cnt; t += BS) {
+    const int sites = min(BS, n - i0);
+    for (int t = threadIdx.x; t < sites * W; t += BS) {
         const double v = sd[t];
         if (WD) thd[(size_t)i0 * W + t] = v;
         if (WF) thf[(size_t)i0 * W + t] = (float)v;
+    }
+    for (int t = threadIdx.x; t < sites * kRecWords; t += BS) {
+        const int site = t / kRecWords, w = t % kRecWords;
+        const size_t o = (size_t)i0 * kRecWords + t;
+        if (w < 6 * P) {  // axis w / 2P, order (w / P) % 2
+            const double v = sd[site * W + w / (2 * P) * 4 * P + w % (2 * P)];
+            if (WD) recd[o] = v;
+            if (WF) recf[o] = (float)v;
+        } else {
+            const unsigned long long k = sk[site];
+            if (WD) recd[o] = w == 6 * P ? __longlong_as_double((long long)k) : 0.0;
+            if (WF) recf[o] = __uint_as_float(w == 6 * P ? (unsigned)k : (unsigned)(k >> 32));
+        }
     }
 }
 
