@@ -92,6 +92,7 @@ struct Pme {
     typename Cplx<R>::type* zg = nullptr;    // [K1 K2 K3] spreading grid, zero between uses
     typename Cplx<R>::type* zq = nullptr;    // [K1 K2 K3] convolved potentials (d + i p)
     R* Gfull = nullptr;                      // [K1 K2 K3] influence function on the full grid
+    double* bsmod = nullptr;                 // [K1 + K2 + K3] B-spline moduli
     double infl_box[6] = {0, 0, 0, 0, 0, 0};
     size_t G = 0, Gc = 0;
 };
@@ -419,49 +420,20 @@ void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
         // in-place complex transform of the dipole grid (d + i p)
         CKFFT(cufftPlan3d(&pm.zplan, K1, K2, K3, CufftTypes<R>::c2c));
         CKFFT(cufftSetStream(pm.zplan, ctx->st));
+        std::vector<double> mod, axis;
+        for (int a = 0; a < 3; a++) {
+            bsmod_axis(ctx->K[a], kOrder, axis);
+            mod.insert(mod.end(), axis.begin(), axis.end());
+        }
+        upload(ctx, pm.bsmod, mod.data(), mod.size());
         pm.ready = true;
     }
     if (!std::equal(ctx->box, ctx->box + 6, pm.infl_box)) {
-        std::vector<double> b1, b2, b3;
-        bsmod_axis(K1, kOrder, b1);
-        bsmod_axis(K2, kOrder, b2);
-        bsmod_axis(K3, kOrder, b3);
-        const double V = ctx->vol;
-        const double pref = 1.0 / (kPi * V), a2 = ctx->aewald * ctx->aewald;
-        const Frac& F = ctx->frac;  // reciprocal vector b_j = (column j of F.m) / K_j
-        std::vector<R> h(pm.Gc);
         const int K3h = K3 / 2 + 1;
-        for (int a = 0; a < K1; a++)
-            for (int b = 0; b < K2; b++)
-                for (int c = 0; c < K3h; c++) {
-                    size_t id = ((size_t)a * K2 + b) * K3h + c;
-                    if (a == 0 && b == 0 && c == 0) { h[id] = 0; continue; }
-                    int ma = a <= K1 / 2 ? a : a - K1, mb = b <= K2 / 2 ? b : b - K2, mc = c;
-                    const double fa = (double)ma / K1, fb = (double)mb / K2, fc = (double)mc / K3;
-                    double hx = F.m[0][0] * fa + F.m[0][1] * fb + F.m[0][2] * fc;
-                    double hy = F.m[1][0] * fa + F.m[1][1] * fb + F.m[1][2] * fc;
-                    double hz = F.m[2][0] * fa + F.m[2][1] * fb + F.m[2][2] * fc;
-                    if (!F.general) { hx = ma / ctx->box[0]; hy = mb / ctx->box[1]; hz = mc / ctx->box[2]; }
-                    double h2 = hx * hx + hy * hy + hz * hz;
-                    h[id] = (R)(pref * exp(-kPi * kPi * h2 / a2) / h2 / (b1[a] * b2[b] * b3[c]));
-                    // octahedron and dodecahedron: the cell's lattice is the
-                    // prism's plus its body-centring translation (half of every
-                    // edge), so its reciprocal vectors are the prism's with an
-                    // even index sum; the others cancel between the two halves
-                    if (ctx->bx.shape >= 3 && ((ma + mb + mc) & 1)) h[id] = 0;
-                }
-        CK(cudaMemcpy(pm.infl, h.data(), sizeof(R) * pm.Gc, cudaMemcpyHostToDevice));
-        // the same function on the full grid (even: G(m) = G(-m))
-        std::vector<R> hf(pm.G);
-        for (int a = 0; a < K1; a++)
-            for (int b = 0; b < K2; b++)
-                for (int c = 0; c < K3; c++) {
-                    const int a2 = a == 0 ? 0 : K1 - a, b2 = b == 0 ? 0 : K2 - b;
-                    // c > K3/2: G(a,b,c) = G(-a,-b,K3-c), held in the half-complex layout
-                    hf[((size_t)a * K2 + b) * K3 + c] =
-                        c < K3h ? h[((size_t)a * K2 + b) * K3h + c] : h[((size_t)a2 * K2 + b2) * K3h + (K3 - c)];
-                }
-        CK(cudaMemcpy(pm.Gfull, hf.data(), sizeof(R) * pm.G, cudaMemcpyHostToDevice));
+        k_influence<R><<<dim3((unsigned)((K3h + 31) / 32), (unsigned)((K2 + 7) / 8), (unsigned)K1), dim3(32, 8), 0,
+                         ctx->st>>>(make_int3(K1, K2, K3), ctx->frac, ctx->bx, ctx->vol, ctx->aewald, pm.bsmod, pm.infl,
+                                    pm.Gfull);
+        CK(cudaGetLastError());  // set-up of the box, not one of an evaluation's launches
         std::copy(ctx->box, ctx->box + 6, pm.infl_box);
     }
 }
@@ -471,7 +443,7 @@ void pme_destroy(Pme<R>& pm) {
     cufftHandle* hs[3] = {&pm.f1, &pm.i1, &pm.zplan};
     for (int k = 0; k < 3; k++)
         if (*hs[k]) { cufftDestroy(*hs[k]); *hs[k] = 0; }
-    dfree(pm.zg); dfree(pm.zq); dfree(pm.Gfull);
+    dfree(pm.zg); dfree(pm.zq); dfree(pm.Gfull); dfree(pm.bsmod);
     dfree(pm.grid); dfree(pm.phig); dfree(pm.cgrid); dfree(pm.infl); dfree(pm.theta); dfree(pm.k0); dfree(pm.rec);
     pm.ready = false;
 }
@@ -1555,6 +1527,27 @@ void enqueue_back(amg_ctx* ctx, cudaStream_t s, int flags) {
     CK(cudaEventRecord(ctx->ev[4], s));
 }
 
+// Makes `graph` (consumed) the executable graph `exec`.  A graph captured
+// again with the same nodes -- another box: kernel parameters only, those of
+// the loop body included -- updates the executable one in place, 20 us
+// instead of the 1.3 ms of destroying it and instantiating another (111
+// nodes); other flags or grids give other nodes and a new instance.
+cudaError_t install_graph(cudaGraphExec_t& exec, cudaGraph_t graph) {
+    cudaError_t e = cudaErrorGraphExecUpdateFailure;
+    if (exec) {
+        cudaGraphExecUpdateResultInfo info;
+        e = cudaGraphExecUpdate(exec, graph, &info);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            cudaGraphExecDestroy(exec);
+            exec = nullptr;
+        }
+    }
+    if (e != cudaSuccess) e = cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+    cudaGraphDestroy(graph);
+    return e;
+}
+
 // Captures the whole evaluation as one CUDA graph: the PCG loop is a
 // conditional WHILE node whose body is one iteration; its last kernel sets
 // the condition from the FP64 residual norms on the device.
@@ -1588,7 +1581,7 @@ bool capture_graph(amg_ctx* ctx, int flags) {
             e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps);
             if (e != cudaSuccess) return fail("capture info", e);
             cudaGraphConditionalHandle h;
-            e = cudaGraphConditionalHandleCreate(&h, graph, 0, 0);
+            e = cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault);
             if (e != cudaSuccess) return fail("conditional handle", e);
             enqueue_predict(ctx, s);
             enqueue_pcg_init<R>(ctx, s, h, 1, true);
@@ -1621,10 +1614,7 @@ bool capture_graph(amg_ctx* ctx, int flags) {
     }
     e = cudaStreamEndCapture(s, &graph);
     if (e != cudaSuccess) return fail("end capture", e);
-    if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-    ctx->gexec = nullptr;
-    e = cudaGraphInstantiate(&ctx->gexec, graph, cudaGraphInstantiateFlagUseNodePriority);
-    cudaGraphDestroy(graph);
+    e = install_graph(ctx->gexec, graph);
     if (e != cudaSuccess) {
         ctx->gexec = nullptr;
         return fail("instantiate", e);
@@ -2266,7 +2256,7 @@ bool capture_adjoint(amg_ctx* ctx) {
         e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps);
         if (e != cudaSuccess) return fail(e);
         cudaGraphConditionalHandle h;
-        e = cudaGraphConditionalHandleCreate(&h, graph, 0, 0);
+        e = cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault);
         if (e != cudaSuccess) return fail(e);
         enqueue_pcg_init<R>(ctx, s, h, 1, true);
         e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps);
@@ -2293,10 +2283,7 @@ bool capture_adjoint(amg_ctx* ctx) {
     }
     e = cudaStreamEndCapture(s, &graph);
     if (e != cudaSuccess) return fail(e);
-    if (ctx->adj_gexec) cudaGraphExecDestroy(ctx->adj_gexec);
-    ctx->adj_gexec = nullptr;
-    e = cudaGraphInstantiate(&ctx->adj_gexec, graph, cudaGraphInstantiateFlagUseNodePriority);
-    cudaGraphDestroy(graph);
+    e = install_graph(ctx->adj_gexec, graph);
     ctx->kcount = k0;
     if (e != cudaSuccess) {
         ctx->adj_gexec = nullptr;

@@ -601,9 +601,49 @@ __global__ void k_kvir_polar(size_t npts, int3 K, Frac F, double c2, double f, i
     block_vir_add(v, vir);
 }
 
-// Multiply the transformed grids by the influence function
+// Influence function
 //   G(m) = exp(-pi^2 |h|^2 / alpha^2) / (pi V |h|^2 bsmod1 bsmod2 bsmod3)
-// precomputed in FP64 on the host (half-complex layout, G(0) = 0).
+// of the current box in FP64, half-complex layout (infl) and on the full grid
+// (full, the even extension G(m) = G(-m)); G(0) = 0.  bsmod: the B-spline
+// moduli of the three axes one after the other.  One thread per half-complex
+// point, which also writes its partner past the half-complex range.  Runs
+// when the box changes (every step under pressure coupling): 54^3 in both
+// precisions took the host 1.8 ms, here 6 us.
+template <class R>
+__global__ void __launch_bounds__(256) k_influence(int3 K, Frac F, Box bx, double vol, double alpha,
+                                                   const double* __restrict__ bsmod, R* __restrict__ infl,
+                                                   R* __restrict__ full) {
+    const int K3h = K.z / 2 + 1;
+    const int c = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y * 8 + threadIdx.y, a = blockIdx.z;
+    if (c >= K3h || b >= K.y) return;
+    const int ma = a <= K.x / 2 ? a : a - K.x, mb = b <= K.y / 2 ? b : b - K.y, mc = c;
+    double g = 0;
+    // octahedron and dodecahedron: the cell's lattice is the prism's plus its
+    // body-centring translation (half of every edge), so its reciprocal
+    // vectors are the prism's with an even index sum; the others cancel
+    // between the two halves
+    const bool absent = bx.shape >= 3 && ((ma + mb + mc) & 1);
+    if ((a || b || c) && !absent) {
+        double hx, hy, hz;
+        if (!F.general) {
+            hx = ma / bx.L[0]; hy = mb / bx.L[1]; hz = mc / bx.L[2];
+        } else {  // reciprocal vector b_j = (column j of F.m) / K_j
+            const double fa = (double)ma / K.x, fb = (double)mb / K.y, fc = (double)mc / K.z;
+            hx = F.m[0][0] * fa + F.m[0][1] * fb + F.m[0][2] * fc;
+            hy = F.m[1][0] * fa + F.m[1][1] * fb + F.m[1][2] * fc;
+            hz = F.m[2][0] * fa + F.m[2][1] * fb + F.m[2][2] * fc;
+        }
+        const double h2 = hx * hx + hy * hy + hz * hz;
+        g = exp(-kPi * kPi * h2 / (alpha * alpha)) / (kPi * vol * h2 * (bsmod[a] * bsmod[K.x + b] * bsmod[K.x + K.y + c]));
+    }
+    infl[((size_t)a * K.y + b) * K3h + c] = (R)g;
+    full[((size_t)a * K.y + b) * K.z + c] = (R)g;
+    if (c > 0 && K.z - c >= K3h)
+        full[((size_t)(a ? K.x - a : 0) * K.y + (b ? K.y - b : 0)) * K.z + (K.z - c)] = (R)g;
+}
+
+// Multiply the transformed grids by the influence function (half-complex
+// layout).
 // The same kernel clears the real spreading grids ([batch][nreal], already
 // consumed by the forward FFT) for the next spreading pass.
 template <class R>
