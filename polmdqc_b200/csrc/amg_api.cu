@@ -33,13 +33,20 @@ namespace {
 constexpr int kOrder = 5;        // B-spline order compiled in (pme.h bseorder default)
 constexpr int kGatherLanes = 4;  // lanes per site in the PME gathers (8: within 3% either way up to 12,288 sites, slower above)
 constexpr int kThreads = 128;
-constexpr int kRbChunks = 8;  // pieces of the gradient read-back
+// Gradient read-back in at most kRbChunks pieces of at least kRbPiece values:
+// a copy costs a few microseconds whatever its size
+constexpr int kRbChunks = 8;
+constexpr size_t kRbPiece = 16384;
 // FP64 accumulators (eacc): em real 0, einter 1, em reciprocal 2, net charge
 // 3, ep 4; the virial's six sums (xx yy zz xy xz yz) of em from kVir and of
 // ep from kVirP
 constexpr int kVir = 8;
 constexpr int kVirP = 14;
 constexpr int kEacc = 20;
+// Status block of an evaluation, one device array so that one copy reads it
+// (in doubles): the accumulators, four counters, the PCG scalars, then two
+// integers (PCG iterations, list overflow); the polarization gradient follows
+constexpr int kStCnt = kEacc, kStScal = kStCnt + 4, kStInt = kStScal + 16, kStatus = 64;
 
 inline unsigned nblk(size_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
@@ -201,16 +208,13 @@ struct amg_ctx {
     // launches outside the PCG loop and per loop iteration
     long long kcount = 0, kmain = 0, kbody = 0, klast = 0;
     char* flushbuf = nullptr;
-    // pinned host staging of one evaluation's read-back (status, scalars,
-    // gradients), filled by asynchronous copies behind one synchronisation
-    struct Readback {
-        int over, iters, over_m;
-        double e[kEacc];
-        unsigned long long c[4];
-        double hs[NSCAL];
-    };
-    Readback* rb = nullptr;
-    double* rb_grad = nullptr;  // [2][3n]
+    // pinned host staging of one evaluation's read-back, filled by
+    // asynchronous copies behind one synchronisation: the status block with
+    // the polarization gradient behind it, as on the device, then the
+    // permanent-multipole gradient
+    double* status = nullptr;       // device [kStatus + 3n]
+    double* rb = nullptr;           // pinned [kStatus + 6n]
+    int* rb_over_m = nullptr;       // pinned: the overflow flag read with the permanent-multipole gradient
     cudaEvent_t rbev[1 + kRbChunks] = {};  // scalars read back, then each gradient piece
     // the permanent-multipole gradient, read back on its own stream while the
     // solve still runs: gm_ready is recorded when the force stream is done
@@ -690,7 +694,6 @@ void ensure_list_buffers(amg_ctx* ctx) {
         dalloc(ctx, ctx->ids, n);
         dalloc(ctx, ctx->sids, n);
         dalloc(ctx, ctx->nnb, n);
-        dalloc(ctx, ctx->overflow, 1);
         dalloc(ctx, ctx->spos, n);
         dalloc(ctx, ctx->rank, n);
         dalloc(ctx, ctx->sdt, n);
@@ -1200,9 +1203,7 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
     enqueue_lists(ctx, r);
     rotate_and_pack<R>(ctx, s);
     if (mixed && iterative(ctx)) rotate_and_pack<double>(ctx, s);
-    k_zero<double><<<1, 32, 0, s>>>(ctx->eacc, kEacc);
-    KCHECK();
-    k_zero<unsigned long long><<<1, 32, 0, s>>>(ctx->cnt, 4);
+    k_zero<double><<<1, 32, 0, s>>>(ctx->status, kStScal);  // accumulators and counters
     KCHECK();
     CK(cudaEventRecord(ctx->erot, s));  // the packed sites for the cell-order copy
     CK(cudaStreamWaitEvent(r, ctx->erot, 0));
@@ -1658,12 +1659,19 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     ctx->want_vir = (flags & AMG_DO_VIRIAL) != 0;
     cudaStream_t st = ctx->st;
     if (!ctx->rb) {
-        CK(cudaMallocHost((void**)&ctx->rb, sizeof(amg_ctx::Readback)));
-        CK(cudaMallocHost((void**)&ctx->rb_grad, sizeof(double) * 6 * (size_t)n));
+        CK(cudaMallocHost((void**)&ctx->rb, sizeof(double) * (kStatus + 6 * (size_t)n)));
+        CK(cudaMallocHost((void**)&ctx->rb_over_m, sizeof(int)));
         for (auto& e : ctx->rbev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         for (auto& e : ctx->rbevm) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     bool dem_added = false;  // the permanent-multipole gradient is in res->dem
+    // the staged status block and gradients, the latter in `pieces` pieces
+    const size_t n3 = 3 * (size_t)n;
+    const int pieces = (int)std::min<size_t>(kRbChunks, std::max<size_t>(1, n3 / kRbPiece));
+    const size_t piece = (n3 + pieces - 1) / pieces;
+    const int* h_int = reinterpret_cast<const int*>(ctx->rb + kStInt);
+    const double* gp = ctx->rb + kStatus;
+    double* gm = ctx->rb + kStatus + n3;
     for (int attempt = 0; attempt < 2; attempt++) {
         ensure_list_buffers(ctx);
         if (iterative(ctx)) ensure_coeff_buffers<R>(ctx, atoms_of<R>(ctx));
@@ -1682,52 +1690,47 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
         }
         if (!graphed) enqueue_eager<R>(ctx, flags);
         ctx->klast = graphed ? -1 : ctx->kcount - kstart;  // graph: completed below from the iteration count
-        // status, scalars and gradients behind one synchronisation
-        amg_ctx::Readback* rb = ctx->rb;
-        CK(cudaMemcpyAsync(&rb->over, ctx->overflow, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(rb->e, ctx->eacc, sizeof(rb->e), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(rb->c, ctx->cnt, sizeof(rb->c), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(rb->hs, ctx->scal, sizeof(double) * NSCAL, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&rb->iters, ctx->iter, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaEventRecord(ctx->rbev[0], st));
-        // the gradients in kRbChunks pieces, each with its event: the host adds
-        // a piece to the caller's arrays while the next one is in flight.  The
-        // permanent-multipole gradient is final once its force stream is done
-        // (gm_ready), so its pieces are copied, and added, beside the solve;
-        // the list-overflow flag, final by then too, is read with them.
-        const size_t n3 = 3 * (size_t)n, piece = (n3 + kRbChunks - 1) / kRbChunks;
+        // status and gradients behind one synchronisation.  The gradients come
+        // in pieces, each with its event: the host adds a piece to the
+        // caller's arrays while the next one is in flight; the first piece of
+        // the polarization gradient comes with the status block before it (5
+        // copies of scalars and 8 pieces whatever the size took 60 us of the
+        // 549 us of a step of 216 waters).  The permanent-multipole
+        // gradient is final once its force stream is done (gm_ready), so its
+        // pieces are copied, and added, beside the solve; the list-overflow
+        // flag, final by then too, is read with them.
         const bool early_m = grad && res->dem;
+        const bool want_p = grad && res->dep && ctx->has_pol;
         if (early_m) {
             CK(cudaStreamWaitEvent(ctx->rbst, ctx->gm_ready, 0));
-            CK(cudaMemcpyAsync(&rb->over_m, ctx->overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx->rbst));
-            for (int k = 0; k < kRbChunks; k++) {
+            CK(cudaMemcpyAsync(ctx->rb_over_m, ctx->overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx->rbst));
+            for (int k = 0; k < pieces; k++) {
                 const size_t a = std::min(n3, k * piece), b = std::min(n3, a + piece);
-                if (b > a)
-                    CK(cudaMemcpyAsync(ctx->rb_grad + a, ctx->grad_m + a, sizeof(double) * (b - a),
-                                       cudaMemcpyDeviceToHost, ctx->rbst));
+                CK(cudaMemcpyAsync(gm + a, ctx->grad_m + a, sizeof(double) * (b - a), cudaMemcpyDeviceToHost,
+                                   ctx->rbst));
                 CK(cudaEventRecord(ctx->rbevm[k], ctx->rbst));
             }
         }
-        for (int k = 0; k < kRbChunks; k++) {
-            const size_t a = std::min(n3, k * piece), b = std::min(n3, a + piece);
-            if (b > a && grad && res->dep && ctx->has_pol)
-                CK(cudaMemcpyAsync(ctx->rb_grad + n3 + a, ctx->grad_p + a, sizeof(double) * (b - a),
-                                   cudaMemcpyDeviceToHost, st));
-            CK(cudaEventRecord(ctx->rbev[1 + k], st));
+        for (int k = 0; k < (want_p ? pieces : 1); k++) {
+            const size_t a = k ? kStatus + std::min(n3, k * piece) : 0;
+            const size_t b = want_p ? kStatus + std::min(n3, (k + 1) * piece) : kStatus;
+            if (b > a)
+                CK(cudaMemcpyAsync(ctx->rb + a, ctx->status + a, sizeof(double) * (b - a), cudaMemcpyDeviceToHost, st));
+            CK(cudaEventRecord(ctx->rbev[k], st));
         }
         if (early_m) {
-            CK(cudaEventSynchronize(ctx->rbevm[0]));  // over_m landed before the first piece
-            if (rb->over_m <= ctx->cap) {
+            CK(cudaEventSynchronize(ctx->rbevm[0]));  // the flag landed before the first piece
+            if (*ctx->rb_over_m <= ctx->cap) {
                 dem_added = true;
-                for (int k = 0; k < kRbChunks; k++) {
+                for (int k = 0; k < pieces; k++) {
                     const size_t a = std::min(n3, k * piece), b = std::min(n3, a + piece);
                     CK(cudaEventSynchronize(ctx->rbevm[k]));
-                    for (size_t q = a; q < b; q++) res->dem[q] += ctx->rb_grad[q];
+                    for (size_t q = a; q < b; q++) res->dem[q] += gm[q];
                 }
             }
         }
         CK(cudaEventSynchronize(ctx->rbev[0]));
-        const int over = rb->over;
+        const int over = h_int[1];
         if (over <= ctx->cap) break;
         CK(cudaStreamSynchronize(st));
         if (attempt == 1) {
@@ -1744,10 +1747,10 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     }
     ctx->graphed_last = ctx->use_graphs && ctx->bounds && ctx->gexec != nullptr;
     // ---- results
-    const double* e = ctx->rb->e;
-    const double* hs = ctx->rb->hs;
-    const unsigned long long* c = ctx->rb->c;
-    int iters = ctx->rb->iters;
+    const double* e = ctx->rb;
+    const double* hs = ctx->rb + kStScal;
+    const unsigned long long* c = reinterpret_cast<const unsigned long long*>(ctx->rb + kStCnt);
+    int iters = h_int[0];
     double eps = 0;
     int status = AMG_OK;
     if (ctx->klast < 0) ctx->klast = ctx->kmain + (long long)iters * ctx->kbody;
@@ -1791,16 +1794,14 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     if (grad) {  // added to the caller's arrays piece by piece as the copies land
         double* dem = dem_added ? nullptr : res->dem;
         double* dep = ctx->has_pol ? res->dep : nullptr;
-        const size_t n3 = 3 * (size_t)n, piece = (n3 + kRbChunks - 1) / kRbChunks;
-        const double* gm = ctx->rb_grad;
-        const double* gp = ctx->rb_grad + n3;
-        for (int k = 0; k < kRbChunks; k++) {
+        for (int k = 0; k < pieces; k++) {
             const size_t a = std::min(n3, k * piece), b = std::min(n3, a + piece);
-            CK(cudaEventSynchronize(ctx->rbev[1 + k]));
+            if (dep) {
+                CK(cudaEventSynchronize(ctx->rbev[k]));
+                for (size_t q = a; q < b; q++) dep[q] += gp[q];
+            }
             if (dem)
                 for (size_t q = a; q < b; q++) dem[q] += gm[q];
-            if (dep)
-                for (size_t q = a; q < b; q++) dep[q] += gp[q];
         }
     }
     if (analysis) {
@@ -1824,9 +1825,11 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     }
     CK(cudaStreamSynchronize(st));
     float ms[4] = {0, 0, 0, 0};
-    for (int k = 0; k < 4; k++)
-        if (cudaEventElapsedTime(&ms[k], ctx->ev[k], ctx->ev[k + 1]) != cudaSuccess) ms[k] = 0;
-    cudaGetLastError();
+    if (!ctx->graphed_last) {  // the phase events exist in the eager path only
+        for (int k = 0; k < 4; k++)
+            if (cudaEventElapsedTime(&ms[k], ctx->ev[k], ctx->ev[k + 1]) != cudaSuccess) ms[k] = 0;
+        cudaGetLastError();
+    }
     ctx->timing[0] = ms[0] + ms[1] + ms[2] + ms[3];
     for (int k = 0; k < 4; k++) ctx->timing[k + 1] = ms[k];
     ctx->have_forward = true;
@@ -1840,7 +1843,7 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
 
 void release(amg_ctx* ctx) {
     if (ctx->rb) { cudaFreeHost(ctx->rb); ctx->rb = nullptr; }
-    if (ctx->rb_grad) { cudaFreeHost(ctx->rb_grad); ctx->rb_grad = nullptr; }
+    if (ctx->rb_over_m) { cudaFreeHost(ctx->rb_over_m); ctx->rb_over_m = nullptr; }
     for (auto& e : ctx->rbev)
         if (e) { cudaEventDestroy(e); e = nullptr; }
     for (auto& e : ctx->rbevm)
@@ -1850,12 +1853,12 @@ void release(amg_ctx* ctx) {
     if (ctx->adj_host) { cudaFreeHost(ctx->adj_host); ctx->adj_host = nullptr; }
     double** dbl[] = {&ctx->pole13, &ctx->pol, &ctx->thole, &ctx->pdamp, &ctx->xyz, &ctx->rp10, &ctx->Ed, &ctx->Ep,
                       &ctx->ud, &ctx->up, &ctx->rd, &ctx->rp, &ctx->zd, &ctx->zp, &ctx->pd, &ctx->pp, &ctx->Apd,
-                      &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->scal, &ctx->eacc, &ctx->grad_m, &ctx->grad_p,
+                      &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->status, &ctx->grad_m,
                       &ctx->trq_m, &ctx->trq_p, &ctx->aem, &ctx->aep, &ctx->phiM, &ctx->phiU, &ctx->phiU4,
                       &ctx->uopt};
     for (double** p : dbl) dfree(*p);
     int** ints[] = {&ctx->zax, &ctx->xax, &ctx->yax, &ctx->axe, &ctx->mol, &ctx->ids, &ctx->sids, &ctx->cstart,
-                    &ctx->cend, &ctx->nbr, &ctx->nnb, &ctx->overflow, &ctx->xoff, &ctx->xidx};
+                    &ctx->cend, &ctx->nbr, &ctx->nnb, &ctx->xoff, &ctx->xidx};
     dfree(ctx->xrange);
     for (int** p : ints) dfree(*p);
     dfree(ctx->keys);
@@ -1864,7 +1867,6 @@ void release(amg_ctx* ctx) {
     dfree(ctx->cnb);
     dfree(ctx->sdt);
     dfree(ctx->spos);
-    dfree(ctx->cnt);
     dfree(ctx->sp);
     if (ctx->cubtmp) cudaFree(ctx->cubtmp);
     ctx->cubtmp = nullptr;
@@ -1884,7 +1886,6 @@ void release(amg_ctx* ctx) {
     }
     if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
     if (ctx->adj_gexec) { cudaGraphExecDestroy(ctx->adj_gexec); ctx->adj_gexec = nullptr; }
-    dfree(ctx->iter);
     dfree(ctx->cont);
     dfree(ctx->blk_done);
     dfree(ctx->flushbuf);
@@ -1981,11 +1982,17 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     ctx->lpa = 8;  // lanes per site (8 measured fastest at 12k and 98k sites)
     if (const char* l = getenv("AMG_LPA")) ctx->lpa = atoi(l);
     if (ctx->lpa != 8 && ctx->lpa != 16 && ctx->lpa != 32) ctx->lpa = 16;
-    dalloc(ctx, ctx->iter, 1);
     dalloc(ctx, ctx->cont, 1);
     dalloc(ctx, ctx->blk_done, 1);
     CK(cudaMemset(ctx->blk_done, 0, sizeof(int)));
-    CK(cudaMemset(ctx->iter, 0, sizeof(int)));
+    dalloc(ctx, ctx->status, kStatus + 3 * (size_t)n);
+    CK(cudaMemset(ctx->status, 0, sizeof(double) * (kStatus + 3 * (size_t)n)));
+    ctx->eacc = ctx->status;
+    ctx->cnt = reinterpret_cast<unsigned long long*>(ctx->status + kStCnt);
+    ctx->scal = ctx->status + kStScal;
+    ctx->iter = reinterpret_cast<int*>(ctx->status + kStInt);
+    ctx->overflow = ctx->iter + 1;
+    ctx->grad_p = ctx->status + kStatus;
     if (ctx->has_pol)
         for (int i = 0; i < n; i++) ctx->npolar += P->polarity[i] > 0;
     if (ctx->poltyp == AMG_POL_OPT) {  // src/md/kpolar.cpp:226-236 restated
@@ -2048,8 +2055,8 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
         dalloc(ctx, ctx->af.p4, 2 * (size_t)n);
     }
     double** vecs[] = {&ctx->Ed, &ctx->Ep, &ctx->ud, &ctx->up, &ctx->rd, &ctx->rp, &ctx->zd, &ctx->zp, &ctx->pd,
-                       &ctx->pp, &ctx->Apd, &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->grad_m, &ctx->grad_p,
-                       &ctx->trq_m, &ctx->trq_p};
+                       &ctx->pp, &ctx->Apd, &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->grad_m, &ctx->trq_m,
+                       &ctx->trq_p};
     for (double** p : vecs) {
         dalloc(ctx, *p, 3 * (size_t)n);
         CK(cudaMemset(*p, 0, sizeof(double) * 3 * n));
@@ -2081,9 +2088,6 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     }
     dalloc(ctx, ctx->aem, n);
     dalloc(ctx, ctx->aep, n);
-    dalloc(ctx, ctx->scal, 16);
-    dalloc(ctx, ctx->eacc, kEacc);
-    dalloc(ctx, ctx->cnt, 4);
     dalloc(ctx, ctx->phiM, 20 * (size_t)n);
     CK(cudaMemset(ctx->phiM, 0, sizeof(double) * 20 * n));
     if (ctx->has_pol) {
