@@ -215,6 +215,7 @@ struct amg_ctx {
     double* status = nullptr;       // device [kStatus + 3n]
     double* rb = nullptr;           // pinned [kStatus + 6n]
     int* rb_over_m = nullptr;       // pinned: the overflow flag read with the permanent-multipole gradient
+    std::vector<double> rb_pole;    // [10n] rotated multipoles on their way to amg_results.rpole
     cudaEvent_t rbev[1 + kRbChunks] = {};  // scalars read back, then each gradient piece
     // the permanent-multipole gradient, read back on its own stream while the
     // solve still runs: gm_ready is recorded when the force stream is done
@@ -1651,6 +1652,17 @@ void enqueue_eager(amg_ctx* ctx, int flags) {
     enqueue_back<R>(ctx, s, flags);
 }
 
+// Touches every page of a caller's output array (writes back what is there)
+// while the GPU works: a freshly allocated array gets its pages then, and not
+// one fault at a time inside the copy that ends the call.
+void touch_pages(double* p, size_t count) {
+    constexpr size_t kPage = 4096 / sizeof(double);
+    if (!p || count < kPage) return;
+    volatile double* v = p;
+    for (size_t k = 0; k < count; k += kPage) v[k] = v[k];
+    v[count - 1] = v[count - 1];
+}
+
 template <class R>
 int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     const int n = ctx->n;
@@ -1717,6 +1729,29 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
             if (b > a)
                 CK(cudaMemcpyAsync(ctx->rb + a, ctx->status + a, sizeof(double) * (b - a), cudaMemcpyDeviceToHost, st));
             CK(cudaEventRecord(ctx->rbev[k], st));
+        }
+        // the host's share while the GPU works: pages of the output arrays, then
+        // the multipoles (final since the front) and the permanent gradient
+        if (want_p) touch_pages(res->dep, n3);
+        if (analysis) touch_pages(res->aem, n);
+        if (analysis && ctx->has_pol) touch_pages(res->aep, n);
+        if ((flags & AMG_DO_DIPOLES) && ctx->has_pol) {
+            touch_pages(res->uind, n3);
+            touch_pages(res->uinp, n3);
+        }
+        if (res->rpole) {
+            touch_pages(res->rpole, 13 * (size_t)n);
+            ctx->rb_pole.resize(10 * (size_t)n);
+            if (!early_m) CK(cudaStreamWaitEvent(ctx->rbst, ctx->gm_ready, 0));
+            CK(cudaMemcpyAsync(ctx->rb_pole.data(), ctx->rp10, sizeof(double) * 10 * n, cudaMemcpyDeviceToHost,
+                               ctx->rbst));
+            CK(cudaStreamSynchronize(ctx->rbst));
+            for (int i = 0; i < n; i++) {
+                const double* m = &ctx->rb_pole[10 * (size_t)i];
+                double* o = res->rpole + 13 * (size_t)i;
+                const double v[13] = {m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[5], m[7], m[8], m[6], m[8], m[9]};
+                std::memcpy(o, v, sizeof(v));
+            }
         }
         if (early_m) {
             CK(cudaEventSynchronize(ctx->rbevm[0]));  // the flag landed before the first piece
@@ -1811,17 +1846,6 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     if ((flags & AMG_DO_DIPOLES) && ctx->has_pol) {
         fetch(res->uind, ctx->ud, 3 * (size_t)n);
         fetch(res->uinp, ctx->up, 3 * (size_t)n);
-    }
-    if (res->rpole) {
-        std::vector<double> r10(10 * (size_t)n);
-        CK(cudaMemcpyAsync(r10.data(), ctx->rp10, sizeof(double) * 10 * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        for (int i = 0; i < n; i++) {
-            const double* m = &r10[10 * (size_t)i];
-            double* o = res->rpole + 13 * (size_t)i;
-            double v[13] = {m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[5], m[7], m[8], m[6], m[8], m[9]};
-            std::memcpy(o, v, sizeof(v));
-        }
     }
     CK(cudaStreamSynchronize(st));
     float ms[4] = {0, 0, 0, 0};
@@ -2516,15 +2540,24 @@ int backward_impl(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* gr) 
     // d_thole [n], d_polarity [n]
     double* h = ctx->adj_host;
     double *hx = h, *hpole = h + n3, *hth = hpole + 13 * (size_t)n, *hpol = hth + n;
-    if (gr->d_xyz) CK(cudaMemcpyAsync(hx, grad, sizeof(double) * n3, cudaMemcpyDeviceToHost, s));
-    if (gr->d_pole) CK(cudaMemcpyAsync(hpole, ctx->adj_dpole, sizeof(double) * 13 * n, cudaMemcpyDeviceToHost, s));
-    if (gr->d_thole) CK(cudaMemcpyAsync(hth, dth, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    if (gr->d_polarity) CK(cudaMemcpyAsync(hpol, dpol, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    host_copy(gr->d_xyz, hx, n3);
-    host_copy(gr->d_pole, hpole, 13 * (size_t)n);
-    host_copy(gr->d_thole, hth, n);
-    host_copy(gr->d_polarity, hpol, n);
+    struct Out {
+        double *dst, *stage;
+        const double* src;
+        size_t count;
+    } outs[4] = {{gr->d_pole, hpole, ctx->adj_dpole, 13 * (size_t)n},
+                 {gr->d_xyz, hx, grad, n3},
+                 {gr->d_thole, hth, dth, (size_t)n},
+                 {gr->d_polarity, hpol, dpol, (size_t)n}};
+    for (int k = 0; k < 4; k++) {
+        const Out& o = outs[k];
+        if (o.dst) CK(cudaMemcpyAsync(o.stage, o.src, sizeof(double) * o.count, cudaMemcpyDeviceToHost, s));
+        CK(cudaEventRecord(ctx->rbev[k], s));
+    }
+    for (const Out& o : outs) touch_pages(o.dst, o.count);
+    for (int k = 0; k < 4; k++) {  // copied out while the next is in flight
+        CK(cudaEventSynchronize(ctx->rbev[k]));
+        host_copy(outs[k].dst, outs[k].stage, outs[k].count);
+    }
     return AMG_OK;
 }
 
@@ -2555,16 +2588,19 @@ int amg_create(const amg_params* params, amg_ctx** out) {
     return AMG_OK;
 }
 
-// true when no value is an infinity or a NaN (exponent bits not all set);
-// branch-free, so the compiler vectorises it
+// true when no value is an infinity or a NaN: 0 x is 0 for every finite x and
+// NaN otherwise, so the sum of the products is 0 or NaN (eight sums side by
+// side, which the compiler turns into vector operations; the exponent test
+// took 200 us for 98,304 sites)
 static bool all_finite(const double* x, size_t count) {
-    uint64_t bad = 0;
-    for (size_t i = 0; i < count; i++) {
-        uint64_t b;
-        std::memcpy(&b, x + i, sizeof b);
-        bad |= (uint64_t)((b & 0x7ff0000000000000ull) == 0x7ff0000000000000ull);
-    }
-    return bad == 0;
+    double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    size_t i = 0;
+    for (; i + 8 <= count; i += 8)
+        for (int k = 0; k < 8; k++) s[k] += 0.0 * x[i + k];
+    for (; i < count; i++) s[0] += 0.0 * x[i];
+    double t = 0;
+    for (int k = 0; k < 8; k++) t += s[k];
+    return t == 0.0;
 }
 
 int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {

@@ -138,9 +138,11 @@ class Result:
     vir: np.ndarray
 
 
-def new_results(n):
-    bufs = {k: np.zeros(3 * n) for k in ("dem", "dep", "uind", "uinp")}
-    bufs.update(aem=np.zeros(n), aep=np.zeros(n), rpole=np.zeros(13 * n))
+def new_results(n, overwritten=()):
+    """amg_results with an array for every output: zeros, or memory as it
+    comes for the names in `overwritten` (arrays the call writes whole)."""
+    sizes = {"dem": 3 * n, "dep": 3 * n, "uind": 3 * n, "uinp": 3 * n, "aem": n, "aep": n, "rpole": 13 * n}
+    bufs = {k: np.empty(m) if k in overwritten else np.zeros(m) for k, m in sizes.items()}
     r = abi.amg_results()
     for k, v in bufs.items():
         setattr(r, k, abi.dptr(v))
@@ -176,6 +178,7 @@ class Engine:
         self.lib = abi.load_library()
         self.params = Params(s, st)
         self.n = s.n
+        self.polarizable = st.poltyp != abi.POL_NONE
         self.ctx = C.c_void_p()
         rc = self.lib.amg_create(C.byref(self.params.struct), C.byref(self.ctx))
         if rc != abi.AMG_OK:
@@ -195,7 +198,12 @@ class Engine:
         self._check(self.lib.amg_set_coords(self.ctx, abi.dptr(xyz), abi.dptr(self.box)), "amg_set_coords")
 
     def forward(self, flags=abi.DO_ENERGY | abi.DO_GRADIENT | abi.DO_DIPOLES) -> Result:
-        r, bufs = new_results(self.n)
+        written = {"rpole"}
+        if flags & abi.DO_ANALYSIS:
+            written |= {"aem", "aep"} if self.polarizable else {"aem"}
+        if flags & abi.DO_DIPOLES and self.polarizable:
+            written |= {"uind", "uinp"}
+        r, bufs = new_results(self.n, written)
         self._check(self.lib.amg_forward(self.ctx, flags, C.byref(r)), "amg_forward")
         return collect(r, bufs, self.n)
 
@@ -209,8 +217,8 @@ class Engine:
 
     def backward(self, d_energy=1.0, d_uind=None, d_uinp=None):
         cot = abi.amg_cotangents(d_energy, abi.dptr(d_uind), abi.dptr(d_uinp))
-        out = {"d_pole": np.zeros(13 * self.n), "d_polarity": np.zeros(self.n),
-               "d_thole": np.zeros(self.n), "d_xyz": np.zeros(3 * self.n)}
+        out = {"d_pole": np.empty(13 * self.n), "d_polarity": np.empty(self.n),
+               "d_thole": np.empty(self.n), "d_xyz": np.empty(3 * self.n)}  # all written whole
         g = abi.amg_param_grads(*(abi.dptr(out[k]) for k in ("d_pole", "d_polarity", "d_thole", "d_xyz")))
         self._check(self.lib.amg_backward(self.ctx, C.byref(cot), C.byref(g)), "amg_backward")
         out["d_pole"] = out["d_pole"].reshape(self.n, 13)
