@@ -8,6 +8,7 @@
 #include "../../include/amoeba_gpu.h"
 #include "kernels_setup.cuh"
 #include "kernels_pme.cuh"
+#include "kernels_fft.cuh"
 #include "kernels_pair.cuh"
 #include "kernels_misc.cuh"
 #include "kernels_adjoint.cuh"
@@ -100,6 +101,11 @@ struct Pme {
     typename Cplx<R>::type* zq = nullptr;    // [K1 K2 K3] convolved potentials (d + i p)
     R* Gfull = nullptr;                      // [K1 K2 K3] influence function on the full grid
     double* bsmod = nullptr;                 // [K1 + K2 + K3] B-spline moduli
+    // the dipole grid's own transform (kernels_fft.cuh), where every size is a
+    // product of two radices
+    bool own_fft = false, big_radix = false;
+    FftAxis<R> fx[3] = {};
+    Cx<R>* twiddles = nullptr;               // the three axes' tables
     double infl_box[6] = {0, 0, 0, 0, 0, 0};
     size_t G = 0, Gc = 0;
 };
@@ -399,6 +405,120 @@ void bsmod_axis(int K, int p, std::vector<double>& out) {
         if (out[m] < 1e-7) out[m] = 0.5 * (out[(m - 1 + K) % K] + out[(m + 1) % K]);
 }
 
+// n = r1 r2 with two of the transform's radices, the more equal the better
+// (a step's threads hold r1, then r2 values each); false if there are none
+bool fft_radices(int n, int& r1, int& r2) {
+    const int set[] = {3, 4, 5, 6, 8, 9, 10, 12, 15, 16};
+    r1 = 0;
+    for (int a : set)
+        for (int b : set)
+            if (a * b == n && a <= b && a > r1) {
+                r1 = a;
+                r2 = b;
+            }
+    return r1 != 0;
+}
+
+// Plans the dipole grid's own transform: tables of twiddles for the three
+// axes; without own_fft (a size that is no product of two radices: a factor
+// of 7 or more, or above 256) the library's transform is used.
+template <class R>
+void fft_prepare(amg_ctx* ctx, Pme<R>& pm) {
+    pm.own_fft = true;
+    pm.big_radix = false;
+    for (int a = 0; a < 3; a++) {
+        FftAxis<R>& x = pm.fx[a];
+        x.n = ctx->K[a];
+        if (!fft_radices(x.n, x.r1, x.r2)) {
+            pm.own_fft = false;
+            return;
+        }
+        pm.big_radix = pm.big_radix || x.r2 > 12;
+    }
+    std::vector<Cx<R>> tw;
+    for (const FftAxis<R>& x : pm.fx)
+        for (int k = 0; k < x.r1; k++)
+            for (int j = 0; j < x.r2; j++) {
+                const double phi = -2 * kPi * ((double)j * k) / x.n;
+                tw.push_back(Cx<R>{(R)std::cos(phi), (R)std::sin(phi)});
+            }
+    upload(ctx, pm.twiddles, tw.data(), tw.size());
+    const Cx<R>* p = pm.twiddles;
+    for (FftAxis<R>& x : pm.fx) {
+        x.tw = p;
+        p += x.n;
+    }
+}
+
+// The convolution zq = backward(G forward(zg)) of the dipole grid on stream s;
+// zg is left at zero.
+template <class R>
+void fft_convolve(amg_ctx* ctx, Pme<R>& pm, cudaStream_t s) {
+    const int K1 = ctx->K[0], K2 = ctx->K[1], K3 = ctx->K[2];
+    Cx<R>* in = reinterpret_cast<Cx<R>*>(pm.zg);
+    Cx<R>* g = reinterpret_cast<Cx<R>*>(pm.zq);
+    auto width = [](const FftAxis<R>& x) { return std::max(x.r1, x.r2); };
+    // lines of a block: as many as are 128 bytes side by side and fit 48 KB of
+    // shared memory (bytes each), or a few less where that leaves none over
+    auto tile = [](int lines, size_t bytes) {
+        const int most = std::max(1, std::min(128 / (int)sizeof(Cx<R>), (int)(49152 / bytes)));
+        const int tiles = (lines + most - 1) / most;
+        return (lines + tiles - 1) / tiles;
+    };
+    auto rows = [&](bool backward, const Cx<R>* from, Cx<R>* clear) {
+        const FftAxis<R>& x = pm.fx[2];
+        const int lines = K1 * K2;
+        const size_t bytes = sizeof(Cx<R>) * x.r1 * (x.r2 | 1);
+        const int T = tile(lines, bytes);
+        auto kern = pm.big_radix ? k_fft_rows<R, true> : k_fft_rows<R, false>;
+        kern<<<nblk(lines, T), dim3(width(x), T), bytes * T, s>>>(x, lines, backward, from, g, clear);
+        KCHECK();
+    };
+    auto columns = [&](bool backward) {
+        const FftAxis<R>& y = pm.fx[1];
+        const size_t bytes = sizeof(Cx<R>) * y.n;
+        const int T = tile(K3, bytes);
+        auto kern = pm.big_radix ? k_fft_strided<R, true, false> : k_fft_strided<R, false, false>;
+        kern<<<dim3(nblk(K3, T), K1), dim3(T, width(y)), bytes * T, s>>>(y, K3, K3, (size_t)K2 * K3, backward, g,
+                                                                        nullptr);
+        KCHECK();
+    };
+    // planes of up to 32 KB (44^2 in FP32): three kernels instead of five.
+    // 24^3: 430 -> 422 us per evaluation, 40^3: 606 -> 592; 54^2 (48 KB) is
+    // level, and larger planes would leave no room for the pair kernels' blocks
+    const size_t plane = sizeof(Cx<R>) * fft_plane_words(pm.fx[2], pm.fx[1]);
+    const bool planes = plane <= 32768;
+    auto both = [&](bool backward, const Cx<R>* from, Cx<R>* clear) {
+        const FftAxis<R>&z = pm.fx[2], &y = pm.fx[1];
+        const int steps = std::max(std::max(K2 * z.r1, K2 * z.r2), std::max(K3 * y.r1, K3 * y.r2));
+        const int threads = std::min(512, (steps + 31) / 32 * 32);
+        auto kern = pm.big_radix ? k_fft_planes<R, true> : k_fft_planes<R, false>;
+        kern<<<K1, threads, plane, s>>>(z, y, backward, from, g, clear);
+        KCHECK();
+    };
+    if (planes) {
+        both(false, in, in);
+    } else {
+        rows(false, in, in);
+        columns(false);
+    }
+    {
+        const FftAxis<R>& x = pm.fx[0];
+        const size_t bytes = sizeof(Cx<R>) * x.n;
+        const int T = tile(K2 * K3, bytes);
+        auto kern = pm.big_radix ? k_fft_strided<R, true, true> : k_fft_strided<R, false, true>;
+        kern<<<nblk((size_t)K2 * K3, T), dim3(T, width(x)), bytes * T, s>>>(
+            x, (size_t)K2 * K3, K2 * K3, 0, false, g, pm.Gfull);
+        KCHECK();
+    }
+    if (planes) {
+        both(true, g, nullptr);
+    } else {
+        columns(true);
+        rows(true, g, nullptr);
+    }
+}
+
 template <class R>
 void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
     const int K1 = ctx->K[0], K2 = ctx->K[1], K3 = ctx->K[2];
@@ -431,6 +551,7 @@ void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
             mod.insert(mod.end(), axis.begin(), axis.end());
         }
         upload(ctx, pm.bsmod, mod.data(), mod.size());
+        fft_prepare(ctx, pm);
         pm.ready = true;
     }
     if (!std::equal(ctx->box, ctx->box + 6, pm.infl_box)) {
@@ -448,7 +569,7 @@ void pme_destroy(Pme<R>& pm) {
     cufftHandle* hs[3] = {&pm.f1, &pm.i1, &pm.zplan};
     for (int k = 0; k < 3; k++)
         if (*hs[k]) { cufftDestroy(*hs[k]); *hs[k] = 0; }
-    dfree(pm.zg); dfree(pm.zq); dfree(pm.Gfull); dfree(pm.bsmod);
+    dfree(pm.zg); dfree(pm.zq); dfree(pm.Gfull); dfree(pm.bsmod); dfree(pm.twiddles);
     dfree(pm.grid); dfree(pm.phig); dfree(pm.cgrid); dfree(pm.infl); dfree(pm.theta); dfree(pm.k0); dfree(pm.rec);
     pm.ready = false;
 }
@@ -875,6 +996,10 @@ void pme_dipole_grids(amg_ctx* ctx, cudaStream_t s, const double* vd, const doub
     if (spread) {
         if (clear) CK(cudaMemsetAsync(pm.zg, 0, sizeof(typename Cplx<R>::type) * pm.G, s));
         spread_dipoles<R>(ctx, s, vd, vp);
+    }
+    if (pm.own_fft && !vir) {  // the virial needs the transform before the convolution
+        fft_convolve(ctx, pm, s);
+        return;
     }
     CKFFT(cufftSetStream(pm.zplan, s));
     CKFFT(CufftTypes<R>::cc(pm.zplan, pm.zg, CUFFT_FORWARD));
@@ -2006,6 +2131,14 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     ctx->lpa = 8;  // lanes per site (8 measured fastest at 12k and 98k sites)
     if (const char* l = getenv("AMG_LPA")) ctx->lpa = atoi(l);
     if (ctx->lpa != 8 && ctx->lpa != 16 && ctx->lpa != 32) ctx->lpa = 16;
+    // k_tu_stored uses next to no shared memory, and an SM divided for that
+    // alone takes no block of the transform beside it until it runs empty
+    // (the y and x passes waited 40 us of its 75 at 32,768 waters): 8% of the
+    // L1 stay shared memory, room for two blocks
+    LPA_DISPATCH(ctx->lpa, {
+        CK(cudaFuncSetAttribute(k_tu_stored<float, L>, cudaFuncAttributePreferredSharedMemoryCarveout, 8));
+        CK(cudaFuncSetAttribute(k_tu_stored<double, L>, cudaFuncAttributePreferredSharedMemoryCarveout, 8));
+    });
     dalloc(ctx, ctx->cont, 1);
     dalloc(ctx, ctx->blk_done, 1);
     CK(cudaMemset(ctx->blk_done, 0, sizeof(int)));

@@ -1,7 +1,9 @@
-"""PME spreading and gathers at grid sizes where a stencil line's pairs of
-points wrap, start at odd places or do not exist (odd sizes), on the smallest
-grids and with a count of sites that fills no block, against the FP64 oracle on
-the same grid, in both precisions (the parity tests' tolerances)."""
+"""PME at the edges of its kernels' sizes, against the FP64 oracle on the same
+grid, in both precisions (the parity tests' tolerances): grids where a stencil
+line's pairs of points wrap, start at odd places or do not exist (odd sizes),
+the smallest grids and a count of sites that fills no block; and the dipole
+grid's transform with every kind of radix, in one kernel per plane or one per
+axis, beside sizes that only the library's transform takes (8, 10, 14, 21)."""
 import numpy as np
 import pytest
 
@@ -13,9 +15,16 @@ pytestmark = pytest.mark.gpu
 FLAGS = abi.DO_ENERGY | abi.DO_GRADIENT | abi.DO_DIPOLES
 
 
-@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
-@pytest.mark.parametrize("nfft", [(8, 9, 8), (10, 8, 9), (12, 15, 14), (21, 16, 27)])
-def test_small_and_odd_grids_match_the_oracle(nfft, prec):
+SMALL = [(8, 9, 8), (10, 8, 9), (12, 15, 14), (21, 16, 27), (9, 12, 15), (16, 30, 25), (50, 45, 48), (16, 36, 75)]
+# grids of 7 to 27 points per Angstrom: in FP64 only (FP32 weights and
+# differences of neighbouring points lose what their tolerance asks for, with
+# any transform)
+FINE = [(64, 16, 144), (50, 81, 45), (16, 160, 240), (256, 15, 16)]
+
+
+@pytest.mark.parametrize("nfft, prec", [(k, p) for k in SMALL for p in (abi.PREC_FP64, abi.PREC_MIXED)] +
+                         [(k, abi.PREC_FP64) for k in FINE])
+def test_grid_sizes_match_the_oracle(nfft, prec):
     s = systems.water_box(27, 9.4, seed=3)
     kw = dict(nfft=nfft, cutoff=4.6)
     o = oracle.forward(s, Settings(precision=abi.PREC_FP64, **kw), tol=1e-11, flags=FLAGS)
