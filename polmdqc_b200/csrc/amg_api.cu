@@ -1218,20 +1218,16 @@ void precondition(amg_ctx* ctx, cudaStream_t s) {
     KCHECK();
 }
 
-// Up to this many sites the PCG direction update and the spreading of p are
-// separate kernels, and the spreading runs beside k_tu_stored (4,096 waters:
-// 3.5% faster per evaluation); above it the fused k_pcg_dir_spread is as fast
-// (32,768 waters) with fewer launches.
-constexpr int kSplitSpreadSites = 65536;
-bool split_spread(const amg_ctx* ctx) { return ctx->ewald && ctx->n <= kSplitSpreadSites; }
-
-// p = z + beta p after the rz scalars were rolled; with Ewald (and above
-// kSplitSpreadSites) fused with the spreading of p for the next matvec
+// p = z + beta p after the rz scalars were rolled; with Ewald fused with the
+// spreading of p for the next matvec, before k_tu_stored starts (as a kernel of
+// its own beside k_tu_stored the spreading waits for its share of the SMs:
+// 216 waters 428 against 410 us per evaluation, 1,500: 590 / 538, 4,096: 820 /
+// 779, 32,768: level)
 template <class R>
 void direction(amg_ctx* ctx, cudaStream_t s) {
     const int n = ctx->n;
     Atoms<R>& A = atoms_of<R>(ctx);
-    if (ctx->ewald && !split_spread(ctx)) {
+    if (ctx->ewald) {
         Pme<R>& pm = pme_of<R>(ctx);
         const int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
         k_pcg_dir_spread<R, kOrder><<<spread_blocks<R>(n), 128, 0, s>>>(n, ctx->zd, ctx->zp, ctx->pd, ctx->pp, ctx->scal, A.p4, pm.rec, K,
@@ -1284,10 +1280,9 @@ void enqueue_pcg_iter(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
     direction<R>(ctx, s);
     // p.Ap: fused into the PME gather with Ewald, a separate pass without
     const bool apart = ctx->ewald;  // real-space field kept apart: the gather overlaps k_tu_stored
-    // split: the direction kernel only updates p; p is spread here, beside
-    // k_tu_stored, into the grid the previous transform left cleared
+    // the direction kernel has spread p
     matvec_stored<R>(ctx, s, A.p4, ctx->pd, ctx->pp, ctx->Apd, ctx->App, ctx->ewald ? ctx->scal + PAP_D : nullptr,
-                     split_spread(ctx), apart, false);
+                     false, apart, false);
     if (!ctx->ewald) {
         k_dot2<<<nblk(n3, 256), 256, 0, s>>>(n3, ctx->pd, ctx->Apd, ctx->pp, ctx->App, ctx->scal + PAP_D,
                                               ctx->scal + PAP_P);
