@@ -196,7 +196,7 @@ struct amg_ctx {
     double cell_volume = 1.0;
     int npolar = 0;
     int *iter = nullptr, *cont = nullptr;
-    int* blk_done = nullptr;  // last-block counter of k_precond and k_pcg_update (back to 0 after every launch)
+    int* blk_done = nullptr;  // last-block counter of k_pcg_update (back to 0 after every launch)
     // OPT: order, copm_k = sum_{j>=k} copt_j, and the perturbation orders
     // u^(k) [K+1][2][3n] followed by one [3n] scratch vector
     int optorder = 0;
@@ -1205,20 +1205,26 @@ double pcg_threshold(const amg_ctx* ctx) {
 constexpr double kPrecDiag = 2.0;
 
 // z = M r for both residual sets from the packed s = alpha r (A.s4); adds
-// r.z to the scalars and (its last block) rolls them for the direction update
+// r.z to the scalars.  Lanes per site: the rows are short (~40 partners), but
+// with few sites a lane's serial share is what the kernel waits for (evaluation
+// of 216 waters with 4 / 8 / 16 lanes: 428, 422, 414 us; 1,500: 590, 583, 584;
+// 32,768: 3.24, 3.28, 3.33 ms).
 template <class R>
 void precondition(amg_ctx* ctx, cudaStream_t s) {
     const int n = ctx->n;
     Atoms<R>& A = atoms_of<R>(ctx);
-    constexpr int L = 4;  // lanes per site: the rows are short
-    const unsigned blocks = (unsigned)std::min<size_t>(nblk((size_t)n * L), (size_t)ctx->num_sms * 8);
-    k_precond<R, L><<<blocks, kThreads, 0, s>>>(n, ctx->sids, ctx->nbru, A.cu0, ctx->cap, ctx->nnbu, ctx->xoff, A.s4,
-                                                ctx->pol, kPrecDiag, ctx->rd, ctx->rp, ctx->zd, ctx->zp, ctx->scal,
-                                                ctx->blk_done);
+    auto launch = [&](auto kern, int lanes) {
+        const unsigned blocks = (unsigned)std::min<size_t>(nblk((size_t)n * lanes), (size_t)ctx->num_sms * 8);
+        kern<<<blocks, kThreads, 0, s>>>(n, ctx->sids, ctx->nbru, A.cu0, ctx->cap, ctx->nnbu, ctx->xoff, A.s4, ctx->pol,
+                                         kPrecDiag, ctx->rd, ctx->rp, ctx->zd, ctx->zp, ctx->scal);
+    };
+    if (n <= 2048) launch(k_precond<R, 16>, 16);
+    else if (n <= 8192) launch(k_precond<R, 8>, 8);
+    else launch(k_precond<R, 4>, 4);
     KCHECK();
 }
 
-// p = z + beta p after the rz scalars were rolled; with Ewald fused with the
+// p = z + beta p; with Ewald fused with the
 // spreading of p for the next matvec, before k_tu_stored starts (as a kernel of
 // its own beside k_tu_stored the spreading waits for its share of the SMs:
 // 216 waters 428 against 410 us per evaluation, 1,500: 590 / 538, 4,096: 820 /
@@ -1263,7 +1269,7 @@ void enqueue_pcg_init(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
                                                ctx->zd, ctx->zp, ctx->scal, ctx->sparse_prec ? A.s4 : nullptr,
                                                ctx->rank);
     KCHECK();
-    k_pcg_control<<<1, 1, 0, s>>>(ctx->scal, ctx->iter, pcg_threshold(ctx), ctx->politer, 1, 0, h, use_handle,
+    k_pcg_control<<<1, 1, 0, s>>>(ctx->scal, ctx->iter, pcg_threshold(ctx), ctx->politer, 1, h, use_handle,
                                   ctx->cont);
     KCHECK();
 }
@@ -1294,7 +1300,7 @@ void enqueue_pcg_iter(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
                                                  ctx->sparse_prec ? A.s4 : nullptr, ctx->rank,
                                                  apart ? ctx->Fd : nullptr, apart ? ctx->Fp : nullptr,
                                                  ctx->blk_done, ctx->iter, pcg_threshold(ctx), ctx->politer,
-                                                 ctx->sparse_prec ? 0 : 1, h, use_handle, ctx->cont);
+                                                 h, use_handle, ctx->cont);
     KCHECK();
 }
 

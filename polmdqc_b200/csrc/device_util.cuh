@@ -59,6 +59,27 @@ __device__ __forceinline__ void block_sum_add(double v, double* out) {
     __syncthreads();
 }
 
+// the same for two sums at once, added to out[0] and out[1]
+__device__ __forceinline__ void block_sum_add2(double u, double v, double* out) {
+    __shared__ double part[2][32];
+    u = warp_sum(u);
+    v = warp_sum(v);
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) {
+        part[0][w] = u;
+        part[1][w] = v;
+    }
+    __syncthreads();
+    if (w == 0) {
+        int nw = (blockDim.x + 31) >> 5;
+        double s = warp_sum(lane < nw ? part[0][lane] : 0.0);
+        double t = warp_sum(lane < nw ? part[1][lane] : 0.0);
+        if (lane == 0 && s != 0.0) atomicAdd(out, s);
+        if (lane == 0 && t != 0.0) atomicAdd(out + 1, t);
+    }
+    __syncthreads();
+}
+
 __device__ __forceinline__ void block_sum_add_ll(long long v, unsigned long long* out) {
     __shared__ long long part[32];
     v = warp_sum(v);

@@ -287,35 +287,34 @@ __device__ __forceinline__ void row_apply(const int* __restrict__ idx, const R4<
     }
 }
 
-// PCG scalars: rz (current), p.Ap, rz of the next iteration, r.r, and the
-// previous rz for the direction update
-enum Scal { RZ_D = 0, RZ_P, PAP_D, PAP_P, RZN_D, RZN_P, RR_D, RR_P, RZO_D, RZO_P, NSCAL };
-
-// rz_old <- rz, rz <- rz_new (cleared): the scalars of the direction update
-// p = z + (rz / rz_old) p that follows (rz_old = 0 on the first iteration
-// gives p = z)
-__device__ __forceinline__ void pcg_roll(double* __restrict__ scal) {
-    scal[RZO_D] = scal[RZ_D];
-    scal[RZO_P] = scal[RZ_P];
-    scal[RZ_D] = scal[RZN_D];
-    scal[RZ_P] = scal[RZN_P];
-    scal[RZN_D] = scal[RZN_P] = 0;
-}
+// PCG scalars, both sets of each: rz of the last iteration, p.Ap, rz of this
+// one (summed by the sparse preconditioner, or by the update before it), r.r,
+// and the diagonal preconditioner's rz of the next iteration
+enum Scal { RZ_D = 0, RZ_P, PAP_D, PAP_P, RZN_D, RZN_P, RR_D, RR_P, RZX_D, RZX_P, NSCAL };
 
 // PCG control (one thread), after the residual update: counts the iteration,
 // decides whether to continue (residual above threshold and fewer than
 // politer iterations) and, inside a captured graph, sets the WHILE node's
 // condition.  `first` marks the decision taken right after the initial
-// residual; `roll` rolls the rz scalars here (diagonal preconditioner, whose
-// z comes with the update; the sparse preconditioner rolls them itself).
+// residual; after an iteration its rz becomes the last one (0 before the
+// first, which gives p = z), and the sum of the next starts from what the
+// diagonal preconditioner has added already (0 with the sparse one).  Rolling
+// the scalars here and not at the end of the preconditioner spares that kernel
+// its wait for every block's sum.
 // The loop body starts with the preconditioner and the direction update, so
 // an iteration that meets the threshold ends the loop without them.
 __device__ __forceinline__ void pcg_decide(double* __restrict__ scal, int* __restrict__ iter, double thr2, int maxit,
-                                           int first, int roll, cudaGraphConditionalHandle h, int use_handle,
+                                           int first, cudaGraphConditionalHandle h, int use_handle,
                                            int* __restrict__ cont_out) {
     int it = first ? 0 : *iter + 1;
     *iter = it;
-    if (!first && roll) pcg_roll(scal);
+    if (!first) {
+        scal[RZ_D] = scal[RZN_D];
+        scal[RZ_P] = scal[RZN_P];
+        scal[RZN_D] = scal[RZX_D];
+        scal[RZN_P] = scal[RZX_P];
+        scal[RZX_D] = scal[RZX_P] = 0;
+    }
     double e2 = fmax(scal[RR_D], scal[RR_P]);
     int cont = (e2 > thr2) && (it < maxit);
     *cont_out = cont;

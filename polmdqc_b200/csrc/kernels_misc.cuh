@@ -67,8 +67,8 @@ __global__ void k_zero(T* __restrict__ p, size_t n) {
 
 
 __global__ void k_pcg_control(double* __restrict__ scal, int* __restrict__ iter, double thr2, int maxit, int first,
-                              int roll, cudaGraphConditionalHandle h, int use_handle, int* __restrict__ cont_out) {
-    pcg_decide(scal, iter, thr2, maxit, first, roll, h, use_handle, cont_out);
+                              cudaGraphConditionalHandle h, int use_handle, int* __restrict__ cont_out) {
+    pcg_decide(scal, iter, thr2, maxit, first, h, use_handle, cont_out);
 }
 
 // r = E - A u and rr.  Diagonal preconditioner (s4 null): z = alpha r and
@@ -102,12 +102,8 @@ __global__ void k_pcg_init(int n, const double* __restrict__ Ed, const double* _
             s4[2 * rank[i] + 1] = make_r4<R>((R)sv[3], (R)sv[4], (R)sv[5], R(0));
         }
     }
-    if (!s4) {
-        block_sum_add(rzd, scal + RZ_D);
-        block_sum_add(rzp, scal + RZ_P);
-    }
-    block_sum_add(rrd, scal + RR_D);
-    block_sum_add(rrp, scal + RR_P);
+    if (!s4) block_sum_add2(rzd, rzp, scal + RZN_D);
+    block_sum_add2(rrd, rrp, scal + RR_D);
 }
 
 __global__ void k_dot2(int n3, const double* __restrict__ a1, const double* __restrict__ b1,
@@ -133,13 +129,13 @@ __global__ void k_pcg_update(int n, const double* __restrict__ pol, const double
                              double* __restrict__ zp, double* __restrict__ scal, R4<R>* __restrict__ s4,
                              const int* __restrict__ rank, const double* __restrict__ Fd,
                              const double* __restrict__ Fp, int* __restrict__ done, int* __restrict__ iter,
-                             double thr2, int maxit, int roll, cudaGraphConditionalHandle h, int use_handle,
+                             double thr2, int maxit, cudaGraphConditionalHandle h, int use_handle,
                              int* __restrict__ cont_out) {
     // one thread per vector component q = 3i + c (the site loop had too few
     // threads in flight for its chains of dependent loads), blocks striding
     // over the components so that few blocks add to the scalars
-    double ad = scal[PAP_D] != 0 ? scal[RZ_D] / scal[PAP_D] : 0.0;
-    double ap = scal[PAP_P] != 0 ? scal[RZ_P] / scal[PAP_P] : 0.0;
+    double ad = scal[PAP_D] != 0 ? scal[RZN_D] / scal[PAP_D] : 0.0;
+    double ap = scal[PAP_P] != 0 ? scal[RZN_P] / scal[PAP_P] : 0.0;
     double rzd = 0, rzp = 0, rrd = 0, rrp = 0;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 3 * n; q += gridDim.x * blockDim.x) {
         const int i = q / 3, c = q - 3 * (q / 3);
@@ -160,12 +156,8 @@ __global__ void k_pcg_update(int n, const double* __restrict__ pol, const double
         }
         rrd += r1 * r1; rrp += r2 * r2;
     }
-    if (!s4) {
-        block_sum_add(rzd, scal + RZN_D);
-        block_sum_add(rzp, scal + RZN_P);
-    }
-    block_sum_add(rrd, scal + RR_D);
-    block_sum_add(rrp, scal + RR_P);
+    if (!s4) block_sum_add2(rzd, rzp, scal + RZX_D);
+    block_sum_add2(rrd, rrp, scal + RR_D);
     // the last block to finish (counted in *done, which it resets) takes the
     // control decision: every block has added its r.r by then
     if (threadIdx.x == 0) {
@@ -173,15 +165,15 @@ __global__ void k_pcg_update(int n, const double* __restrict__ pol, const double
         if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
             __threadfence();
             *done = 0;
-            pcg_decide(scal, iter, thr2, maxit, 0, roll, h, use_handle, cont_out);
+            pcg_decide(scal, iter, thr2, maxit, 0, h, use_handle, cont_out);
         }
     }
 }
 
-// beta = rz / rz_old after the scalars were rolled (0 on the first iteration)
+// beta = rz of this iteration over the last one's (0 on the first iteration)
 __device__ __forceinline__ void pcg_beta(const double* __restrict__ scal, double& bd, double& bp) {
-    bd = scal[RZO_D] != 0 ? scal[RZ_D] / scal[RZO_D] : 0.0;
-    bp = scal[RZO_P] != 0 ? scal[RZ_P] / scal[RZO_P] : 0.0;
+    bd = scal[RZ_D] != 0 ? scal[RZN_D] / scal[RZ_D] : 0.0;
+    bp = scal[RZ_P] != 0 ? scal[RZN_P] / scal[RZ_P] : 0.0;
 }
 
 // p = z + beta p; p = z when beta = 0 (the first direction, whose old p is
@@ -190,7 +182,7 @@ __device__ __forceinline__ double pcg_dir_value(double z, double beta, double p)
     return beta != 0 ? z + beta * p : z;
 }
 
-// p = z + beta p and its R4 copy (after the rz scalars were rolled)
+// p = z + beta p and its R4 copy
 template <class R>
 __global__ void k_pcg_dir(int n, const double* __restrict__ zd, const double* __restrict__ zp,
                           double* __restrict__ pd, double* __restrict__ pp, const double* __restrict__ scal,
@@ -211,7 +203,7 @@ __global__ void k_pcg_dir(int n, const double* __restrict__ zd, const double* __
     p4[2 * rank[i] + 1] = make_r4<R>((R)b[0], (R)b[1], (R)b[2], R(0));
 }
 
-// p = z + beta p (after the rz scalars were rolled) fused with the spreading of
+// p = z + beta p fused with the spreading of
 // p into the complex grid zg for the next matvec (zg holds the cleared grid
 // left by the previous transform), in the layout of k_spread_dipoles: FP32,
 // kLineSites sites per block of 128 threads and one z-line per thread; FP64,

@@ -428,10 +428,7 @@ __global__ void __launch_bounds__(128) k_tu_stored(int n, const int* __restrict_
             }
         }
     }
-    if (vAv) {
-        block_sum_add(dd, vAv);
-        block_sum_add(dp, vAv + 1);
-    }
+    if (vAv) block_sum_add2(dd, dp, vAv);
 }
 
 // ------------------------------------------------------------ scaled pairs
@@ -578,9 +575,8 @@ __global__ void k_scaled_coeffs(int np, const ScaledPair* __restrict__ sp, const
 // pairs within usolvcut, then the scaled partners; nbru holds the partners'
 // positions in cell order).  Adds r.z of both sets to scal[RZN_D..RZN_P].
 // Blocks stride over the sites (a grid of a few blocks per SM), so each block
-// adds its r.z once; the last block to finish (counted in *done, which it
-// resets) then rolls the PCG scalars (rz_old <- rz <- r.z) for the direction
-// update that follows.
+// adds its r.z once.  Bound by memory latency (chains of count, index, vector):
+// with few sites more lanes take a row at once (see precondition).
 template <class R, int LPA>
 __global__ void __launch_bounds__(128) k_precond(int n, const int* __restrict__ order, const int* __restrict__ nbru, const R4<R>* __restrict__ cu0,
                                                  int cap, const int* __restrict__ nnbu,
@@ -588,7 +584,7 @@ __global__ void __launch_bounds__(128) k_precond(int n, const int* __restrict__ 
                                                  const double* __restrict__ pol, double wdiag,
                                                  const double* __restrict__ rd, const double* __restrict__ rp,
                                                  double* __restrict__ zd, double* __restrict__ zp,
-                                                 double* __restrict__ scal, int* __restrict__ done) {
+                                                 double* __restrict__ scal) {
     const int lane = threadIdx.x % LPA, per_block = blockDim.x / LPA;
     double rzd = 0, rzp = 0;
     for (int g0 = blockIdx.x * per_block; g0 < n; g0 += gridDim.x * per_block) {
@@ -616,16 +612,7 @@ __global__ void __launch_bounds__(128) k_precond(int n, const int* __restrict__ 
             }
         }
     }
-    block_sum_add(rzd, scal + RZN_D);
-    block_sum_add(rzp, scal + RZN_P);
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-            __threadfence();
-            *done = 0;
-            pcg_roll(scal);
-        }
-    }
+    block_sum_add2(rzd, rzp, scal + RZN_D);
 }
 
 // scaled pairs' contribution to em, its gradient and the torques (both

@@ -485,10 +485,7 @@ __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx
             else dotd += dot;
         }
     }
-    if (vAv) {
-        block_sum_add(dotd, vAv);
-        block_sum_add(dotp, vAv + 1);
-    }
+    if (vAv) block_sum_add2(dotd, dotp, vAv);
 }
 
 // out = G . g on the transformed complex dipole grid (G real, on the full
