@@ -88,8 +88,8 @@ struct CufftTypes<double> {
 template <class R>
 struct Pme {
     bool ready = false;
-    R* grid = nullptr;                       // [2][K1 K2 K3] spreading grids (kept zeroed)
-    R* phig = nullptr;                       // [2][K1 K2 K3] convolved potential grids
+    R* grid = nullptr;                       // [K1 K2 K3] spreading grid, zero between uses
+    R* phig = nullptr;                       // [K1 K2 K3] convolved potential grid
     typename CufftTypes<R>::C* cgrid = nullptr;  // [2][K1 K2 (K3/2+1)]
     R* infl = nullptr;                       // [K1 K2 (K3/2+1)]
     R* theta = nullptr;                      // [n][3][4][P]
@@ -170,8 +170,7 @@ struct amg_ctx {
     double4* spos = nullptr;  // coordinates in cell order
     // vectors
     double *Ed = nullptr, *Ep = nullptr, *ud = nullptr, *up = nullptr, *rd = nullptr, *rp = nullptr, *zd = nullptr,
-           *zp = nullptr, *pd = nullptr, *pp = nullptr, *Apd = nullptr, *App = nullptr, *Fd = nullptr, *Fp = nullptr,
-           *resd = nullptr;
+           *zp = nullptr, *pd = nullptr, *pp = nullptr, *Apd = nullptr, *App = nullptr, *Fd = nullptr, *Fp = nullptr;
     double *scal = nullptr, *eacc = nullptr;  // eacc: [kEacc]
     bool want_vir = false;                    // this evaluation adds the virial (eacc + kVir, + kVirP)
     bool have_vir = false;
@@ -525,9 +524,9 @@ void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
     if (!pm.ready) {
         pm.G = (size_t)K1 * K2 * K3;
         pm.Gc = (size_t)K1 * K2 * (K3 / 2 + 1);
-        dalloc(ctx, pm.grid, 2 * pm.G);
-        dalloc(ctx, pm.phig, 2 * pm.G);
-        CK(cudaMemset(pm.grid, 0, sizeof(R) * 2 * pm.G));
+        dalloc(ctx, pm.grid, pm.G);
+        dalloc(ctx, pm.phig, pm.G);
+        CK(cudaMemset(pm.grid, 0, sizeof(R) * pm.G));  // k_convolve leaves it clear
         dalloc(ctx, pm.cgrid, 2 * pm.Gc);
         dalloc(ctx, pm.infl, pm.Gc);
         dalloc(ctx, pm.theta, (size_t)ctx->n * 3 * 4 * kOrder);
@@ -1043,7 +1042,7 @@ bool ewald_cells(const amg_ctx* ctx) { return ctx->ewald && ctx->bx.shape != 0; 
 // real-space part gathers from cell-order copies (k_Tu_cells).
 template <class R>
 void matvec(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp, double* Ad, double* Ap,
-            bool cells = false) {
+            bool cells = false, bool finish = true) {
     const int n = ctx->n;
     Atoms<R>& A = atoms_of<R>(ctx);
     k_pack_u<R><<<nblk(n), kThreads, 0, s>>>(n, vd, vp, A.u4, cells ? ctx->rank : nullptr);
@@ -1089,6 +1088,7 @@ void matvec(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp, do
         pme_dipoles<R, 4>(ctx, s, vd, vp, ctx->phiU4);
         join_side(ctx, s);
     }
+    if (!finish) return;  // the fields stay in Fd, Fp and phiU4
     k_matvec_finish<<<nblk(n), kThreads, 0, s>>>(n, vd, vp, ctx->Fd, ctx->Fp, ctx->phiU4, ctx->ewald, self_coef(ctx),
                                                  ctx->pol, Ad, Ap);
     KCHECK();
@@ -1106,35 +1106,6 @@ void build_scaled_coeffs(amg_ctx* ctx, cudaStream_t s) {
         ctx->cap, ctx->rank, ctx->cnb, A.c0, ctx->usolvcut * ctx->usolvcut, sp ? ctx->nnbu : nullptr,
         sp ? ctx->nbru : nullptr, sp ? A.cu0 : nullptr);
     KCHECK();
-}
-
-// pair coefficients of the real-space T for the whole solve (the adjoint's
-// FP64 solve; the forward builds them with the permanent field)
-template <class R>
-void build_tu_coeffs(amg_ctx* ctx, cudaStream_t s) {
-    const int n = ctx->n;
-    Atoms<R>& A = atoms_of<R>(ctx);
-    const bool sp = ctx->sparse_prec;
-    const double u2 = ctx->usolvcut * ctx->usolvcut;
-    int* nbru = sp ? ctx->nbru : nullptr;
-    int* nnbu = sp ? ctx->nnbu : nullptr;
-    R4<R>* cu0 = sp ? A.cu0 : nullptr;
-    LPA_DISPATCH(ctx->lpa, {
-        if (ewald_cells(ctx))
-            k_tu_coeffs<R, true, 8, true><<<nblk((size_t)n * 8), kThreads, 0, s>>>(n, ctx->sids, A.atS, ctx->bx, (R)ctx->aewald,
-                                                                                   ctx->cnb, ctx->cap, ctx->nnb, A.c0,
-                                                                                   (R)u2, nbru, cu0, nnbu);
-        else if (ctx->ewald)
-            k_tu_coeffs<R, true, L><<<nblk((size_t)n * L), kThreads, 0, s>>>(n, ctx->sids, A.atS, ctx->bx, (R)ctx->aewald, ctx->cnb,
-                                                                             ctx->cap, ctx->nnb, A.c0, (R)u2, nbru,
-                                                                             cu0, nnbu);
-        else
-            k_tu_coeffs<R, false, L><<<nblk((size_t)n * L), kThreads, 0, s>>>(n, ctx->sids, A.atS, ctx->bx, (R)0, ctx->cnb, ctx->cap,
-                                                                              ctx->nnb, A.c0, (R)u2, nbru, cu0,
-                                                                              nnbu);
-    });
-    KCHECK();
-    build_scaled_coeffs<R>(ctx, s);
 }
 
 // Blocks of k_tu_stored per SM.  In FP32 9 blocks fit an SM (54 registers),
@@ -1244,33 +1215,35 @@ void direction(amg_ctx* ctx, cudaStream_t s) {
     KCHECK();
 }
 
+// the solve starts from the direct dipoles as the front leaves them: their R4
+// copies and the cleared scalars come with them (k_field_finish)
+bool starts_packed(const amg_ctx* ctx) { return iterative(ctx) && ctx->guess && !ctx->pred; }
+
 // set-up of the solve: r = E - A u0 (with the diagonal preconditioner also
 // z = alpha r and r.z) and the first control decision (continue while
-// rr > threshold and iterations < politer)
+// rr > threshold and iterations < politer).  `packed`: the starting dipoles'
+// R4 copies are there and the scalars cleared.
 template <class R>
-void enqueue_pcg_init(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h, int use_handle,
-                      bool coeffs_built) {
+void enqueue_pcg_init(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h, int use_handle, bool packed) {
     const int n = ctx->n;
     Atoms<R>& A = atoms_of<R>(ctx);
-    if (!ctx->guess) {
-        k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->ud, 3 * (size_t)n);
+    if (!packed) {
+        if (!ctx->guess) {
+            k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->ud, 3 * (size_t)n);
+            KCHECK();
+            k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->up, 3 * (size_t)n);
+            KCHECK();
+        }
+        k_zero<double><<<1, 32, 0, s>>>(ctx->scal, NSCAL);
         KCHECK();
-        k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->up, 3 * (size_t)n);
+        k_pack_u<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->ud, ctx->up, A.u4, ctx->rank);  // cell order
         KCHECK();
     }
-    k_zero<double><<<1, 32, 0, s>>>(ctx->scal, NSCAL);
-    KCHECK();
-    if (!coeffs_built) build_tu_coeffs<R>(ctx, s);
-    k_pack_u<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->ud, ctx->up, A.u4, ctx->rank);  // cell order
-    KCHECK();
-    // leaves the dipole grid clear for the direction updates' spreading
     matvec_stored<R>(ctx, s, A.u4, ctx->ud, ctx->up, ctx->Apd, ctx->App);
     k_pcg_init<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->Ed, ctx->Ep, ctx->Apd, ctx->App, ctx->pol, ctx->rd, ctx->rp,
                                                ctx->zd, ctx->zp, ctx->scal, ctx->sparse_prec ? A.s4 : nullptr,
-                                               ctx->rank);
-    KCHECK();
-    k_pcg_control<<<1, 1, 0, s>>>(ctx->scal, ctx->iter, pcg_threshold(ctx), ctx->politer, 1, h, use_handle,
-                                  ctx->cont);
+                                               ctx->rank, ctx->blk_done, ctx->iter, pcg_threshold(ctx), ctx->politer, h,
+                                               use_handle, ctx->cont);
     KCHECK();
 }
 
@@ -1305,13 +1278,27 @@ void enqueue_pcg_iter(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
 }
 
 // FP64 correction sweep: the true residual with every term in FP64, one
-// diagonal-preconditioned step u += alpha r, and the residual norms
-void enqueue_sweep(amg_ctx* ctx, cudaStream_t s) {
-    matvec<double>(ctx, s, ctx->ud, ctx->up, ctx->Apd, ctx->App, true);
-    k_zero<double><<<1, 32, 0, s>>>(ctx->scal + PAP_D, 6);
-    KCHECK();
-    k_correct<<<nblk(ctx->n), kThreads, 0, s>>>(ctx->n, ctx->Ed, ctx->Ep, ctx->Apd, ctx->App, ctx->pol, ctx->ud, ctx->up,
-                                                ctx->resd, ctx->scal);
+// diagonal-preconditioned step u += alpha r, and the residual norms.  An FP64
+// context has the FP64 coefficient rows of its solve (24,044 sites: 49 us
+// streamed against 75 computed on the fly).  With grad (the forward of
+// precision R) k_correct also prepares the force kernels' dipoles and
+// accumulators.
+template <class R>
+void enqueue_sweep(amg_ctx* ctx, cudaStream_t s, bool forward, bool grad) {
+    const int n = ctx->n;
+    const bool stored = sizeof(R) == 8;
+    if (stored) {
+        k_pack_u<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->ud, ctx->up, atoms_of<R>(ctx).u4, ctx->rank);
+        KCHECK();
+        matvec_stored<R>(ctx, s, atoms_of<R>(ctx).u4, ctx->ud, ctx->up, ctx->Apd, ctx->App);
+    } else {
+        matvec<double>(ctx, s, ctx->ud, ctx->up, ctx->Apd, ctx->App, true, false);
+    }
+    k_correct<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->Ed, ctx->Ep, stored ? ctx->Apd : nullptr,
+                                              stored ? ctx->App : nullptr, ctx->Fd, ctx->Fp, ctx->phiU4, ctx->ewald,
+                                              self_coef(ctx), ctx->pol, ctx->ud, ctx->up, ctx->scal,
+                                              forward ? atoms_of<R>(ctx).u4 : nullptr, ctx->rank,
+                                              grad ? ctx->grad_p : nullptr, grad ? ctx->trq_p : nullptr);
     KCHECK();
 }
 
@@ -1335,7 +1322,6 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
     cudaStream_t r = fork_side(ctx, s);
     enqueue_lists(ctx, r);
     rotate_and_pack<R>(ctx, s);
-    if (mixed && iterative(ctx)) rotate_and_pack<double>(ctx, s);
     k_zero<double><<<1, 32, 0, s>>>(ctx->status, kStScal);  // accumulators and counters
     KCHECK();
     CK(cudaEventRecord(ctx->erot, s));  // the packed sites for the cell-order copy
@@ -1344,14 +1330,6 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
     KCHECK();
     if (ctx->ewald) {
         pme_stencils<R>(ctx, s, mixed && iterative(ctx));  // FP64 ones too for the sweep
-        Pme<R>& pm = pme_of<R>(ctx);
-        k_zero<R><<<nblk(2 * pm.G, 256), 256, 0, s>>>(pm.grid, 2 * pm.G);
-        KCHECK();
-        if (mixed && iterative(ctx)) {
-            Pme<double>& pd = pme_of<double>(ctx);
-            k_zero<double><<<nblk(2 * pd.G, 256), 256, 0, s>>>(pd.grid, 2 * pd.G);
-            KCHECK();
-        }
     }
     CK(cudaEventRecord(ctx->ev[1], s));
     Atoms<R>& A = atoms_of<R>(ctx);
@@ -1391,8 +1369,9 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
     if (ctx->ewald) pme_mpole<R>(ctx, s, ctx->want_vir ? ctx->eacc + kVir : nullptr);
     join_side(ctx, s);
     if (ctx->has_pol) {
-        k_field_finish<<<nblk(n), kThreads, 0, s>>>(n, ctx->phiM, ctx->ewald, ctx->rp10, self_coef(ctx), ctx->pol, ctx->Ed,
-                                                    ctx->Ep, ctx->ud, ctx->up);
+        k_field_finish<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->phiM, ctx->ewald, ctx->rp10, self_coef(ctx), ctx->pol,
+                                                       ctx->Ed, ctx->Ep, ctx->ud, ctx->up,
+                                                       starts_packed(ctx) ? A.u4 : nullptr, ctx->rank, ctx->scal);
         KCHECK();
     }
     CK(cudaEventRecord(ctx->ev[2], s));
@@ -1606,7 +1585,7 @@ void enqueue_back(amg_ctx* ctx, cudaStream_t s, int flags) {
     const R aew = (R)ctx->aewald;
     const int mutual = ctx->poltyp == AMG_POL_MUTUAL;
     CK(cudaEventRecord(ctx->ev[3], s));
-    if (polgrad) {
+    if (polgrad && !iterative(ctx)) {  // after a solve the correction sweep has done this
         k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->grad_p, 3 * (size_t)n);
         KCHECK();
         k_zero<double><<<nblk(3 * n, 256), 256, 0, s>>>(ctx->trq_p, 3 * (size_t)n);
@@ -1725,7 +1704,7 @@ bool capture_graph(amg_ctx* ctx, int flags) {
             e = cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault);
             if (e != cudaSuccess) return fail("conditional handle", e);
             enqueue_predict(ctx, s);
-            enqueue_pcg_init<R>(ctx, s, h, 1, true);
+            enqueue_pcg_init<R>(ctx, s, h, 1, starts_packed(ctx));
             e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps);
             if (e != cudaSuccess) return fail("capture info", e);
             cudaGraphNodeParams cp = {};
@@ -1746,7 +1725,7 @@ bool capture_graph(amg_ctx* ctx, int flags) {
             kb = ctx->kcount - kb0;
             e = cudaStreamEndCapture(ctx->st2, &body);
             if (e != cudaSuccess) return fail("end body capture", e);
-            enqueue_sweep(ctx, s);
+            enqueue_sweep<R>(ctx, s, true, flags & AMG_DO_GRADIENT);
             enqueue_pred_store(ctx, s);
         }
         enqueue_back<R>(ctx, s, flags);
@@ -1777,7 +1756,7 @@ void enqueue_eager(amg_ctx* ctx, int flags) {
     if (ctx->poltyp == AMG_POL_OPT && ctx->npolar > 0) enqueue_opt<R>(ctx, s);
     if (iterative(ctx)) {
         enqueue_predict(ctx, s);
-        enqueue_pcg_init<R>(ctx, s, 0, 0, true);
+        enqueue_pcg_init<R>(ctx, s, 0, 0, starts_packed(ctx));
         int cont = 1;
         while (true) {
             CK(cudaMemcpyAsync(&cont, ctx->cont, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1785,7 +1764,7 @@ void enqueue_eager(amg_ctx* ctx, int flags) {
             if (!cont) break;
             enqueue_pcg_iter<R>(ctx, s, 0, 0);
         }
-        enqueue_sweep(ctx, s);
+        enqueue_sweep<R>(ctx, s, true, flags & AMG_DO_GRADIENT);
         enqueue_pred_store(ctx, s);
     }
     enqueue_back<R>(ctx, s, flags);
@@ -2016,7 +1995,7 @@ void release(amg_ctx* ctx) {
     if (ctx->adj_host) { cudaFreeHost(ctx->adj_host); ctx->adj_host = nullptr; }
     double** dbl[] = {&ctx->pole13, &ctx->pol, &ctx->thole, &ctx->pdamp, &ctx->xyz, &ctx->rp10, &ctx->Ed, &ctx->Ep,
                       &ctx->ud, &ctx->up, &ctx->rd, &ctx->rp, &ctx->zd, &ctx->zp, &ctx->pd, &ctx->pp, &ctx->Apd,
-                      &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->status, &ctx->grad_m,
+                      &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->status, &ctx->grad_m,
                       &ctx->trq_m, &ctx->trq_p, &ctx->aem, &ctx->aep, &ctx->phiM, &ctx->phiU, &ctx->phiU4,
                       &ctx->uopt};
     for (double** p : dbl) dfree(*p);
@@ -2226,7 +2205,7 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
         dalloc(ctx, ctx->af.p4, 2 * (size_t)n);
     }
     double** vecs[] = {&ctx->Ed, &ctx->Ep, &ctx->ud, &ctx->up, &ctx->rd, &ctx->rp, &ctx->zd, &ctx->zp, &ctx->pd,
-                       &ctx->pp, &ctx->Apd, &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->resd, &ctx->grad_m, &ctx->trq_m,
+                       &ctx->pp, &ctx->Apd, &ctx->App, &ctx->Fd, &ctx->Fp, &ctx->grad_m, &ctx->trq_m,
                        &ctx->trq_p};
     for (double** p : vecs) {
         dalloc(ctx, *p, 3 * (size_t)n);
@@ -2433,7 +2412,7 @@ bool capture_adjoint(amg_ctx* ctx) {
         cudaGraphConditionalHandle h;
         e = cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault);
         if (e != cudaSuccess) return fail(e);
-        enqueue_pcg_init<R>(ctx, s, h, 1, true);
+        enqueue_pcg_init<R>(ctx, s, h, 1, false);
         e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, &ndeps);
         if (e != cudaSuccess) return fail(e);
         cudaGraphNodeParams cp = {};
@@ -2452,7 +2431,7 @@ bool capture_adjoint(amg_ctx* ctx) {
         enqueue_pcg_iter<R>(ctx, ctx->st2, h, 1);
         e = cudaStreamEndCapture(ctx->st2, &body);
         if (e != cudaSuccess) return fail(e);
-        enqueue_sweep(ctx, s);
+        enqueue_sweep<R>(ctx, s, false, false);
     } catch (Fail&) {
         return fail(cudaGetLastError());
     }
@@ -2481,7 +2460,7 @@ void adjoint_solve(amg_ctx* ctx, cudaStream_t s) {
             return;
         }
     }
-    enqueue_pcg_init<R>(ctx, s, 0, 0, true);
+    enqueue_pcg_init<R>(ctx, s, 0, 0, false);
     int cont = 1;
     while (true) {
         CK(cudaMemcpyAsync(&cont, ctx->cont, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2489,7 +2468,7 @@ void adjoint_solve(amg_ctx* ctx, cudaStream_t s) {
         if (!cont) break;
         enqueue_pcg_iter<R>(ctx, s, 0, 0);
     }
-    enqueue_sweep(ctx, s);
+    enqueue_sweep<R>(ctx, s, false, false);
 }
 
 // amg_backward: the adjoint solve in the context's precision (above), every

@@ -318,10 +318,9 @@ __device__ __forceinline__ void pcg_decide(double* __restrict__ scal, int* __res
     double e2 = fmax(scal[RR_D], scal[RR_P]);
     int cont = (e2 > thr2) && (it < maxit);
     *cont_out = cont;
-    if (cont) {  // accumulators of the next iteration
-        scal[PAP_D] = scal[PAP_P] = 0;
-        scal[RR_D] = scal[RR_P] = 0;
-    }
+    // accumulators of the next iteration, or of the correction sweep
+    scal[PAP_D] = scal[PAP_P] = 0;
+    scal[RR_D] = scal[RR_P] = 0;
     if (use_handle) cudaGraphSetConditional(h, cont ? 1u : 0u);
 }
 

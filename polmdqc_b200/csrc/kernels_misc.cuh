@@ -7,19 +7,30 @@
 namespace amg {
 
 // Fields from the reciprocal potential (E = -grad phi) and the Ewald self
-// field (4 a^3 / (3 sqrt(pi))) d; then the direct dipoles u = alpha E.
+// field (4 a^3 / (3 sqrt(pi))) d; then the direct dipoles u = alpha E.  With
+// u4 (a PCG that starts from them follows) also their R4 copies in cell order,
+// and the PCG's scalars cleared.
+template <class R>
 __global__ void k_field_finish(int n, const double* __restrict__ phiM, int ewald, const double* __restrict__ rp10,
                                double selfc, const double* __restrict__ pol, double* __restrict__ Ed,
-                               double* __restrict__ Ep, double* __restrict__ ud, double* __restrict__ up) {
+                               double* __restrict__ Ep, double* __restrict__ ud, double* __restrict__ up,
+                               R4<R>* __restrict__ u4, const int* __restrict__ rank, double* __restrict__ scal) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u4 && i < NSCAL) scal[i] = 0;
     if (i >= n) return;
+    double vd[3], vp[3];
     for (int a = 0; a < 3; a++) {
         double add = ewald ? -phiM[20 * (size_t)i + 1 + a] + selfc * rp10[10 * i + 1 + a] : 0.0;
         double ed = Ed[3 * i + a] + add, ep = Ep[3 * i + a] + add;
         Ed[3 * i + a] = ed;
         Ep[3 * i + a] = ep;
-        ud[3 * i + a] = pol[i] * ed;
-        up[3 * i + a] = pol[i] * ep;
+        ud[3 * i + a] = vd[a] = pol[i] * ed;
+        up[3 * i + a] = vp[a] = pol[i] * ep;
+    }
+    if (u4) {
+        const int o = rank[i];
+        u4[2 * o] = make_r4<R>((R)vd[0], (R)vd[1], (R)vd[2], R(0));
+        u4[2 * o + 1] = make_r4<R>((R)vp[0], (R)vp[1], (R)vp[2], R(0));
     }
 }
 
@@ -66,9 +77,20 @@ __global__ void k_zero(T* __restrict__ p, size_t n) {
 }
 
 
-__global__ void k_pcg_control(double* __restrict__ scal, int* __restrict__ iter, double thr2, int maxit, int first,
-                              cudaGraphConditionalHandle h, int use_handle, int* __restrict__ cont_out) {
-    pcg_decide(scal, iter, thr2, maxit, first, h, use_handle, cont_out);
+// the last block to finish (counted in *done, which it resets) takes the PCG's
+// control decision: every block has added its sums by then.  Every block
+// calls it at its end.
+__device__ __forceinline__ void pcg_decide_last(double* __restrict__ scal, int* __restrict__ done,
+                                                int* __restrict__ iter, double thr2, int maxit, int first,
+                                                cudaGraphConditionalHandle h, int use_handle,
+                                                int* __restrict__ cont_out) {
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
+        __threadfence();
+        *done = 0;
+        pcg_decide(scal, iter, thr2, maxit, first, h, use_handle, cont_out);
+    }
 }
 
 // r = E - A u and rr.  Diagonal preconditioner (s4 null): z = alpha r and
@@ -79,7 +101,9 @@ __global__ void k_pcg_init(int n, const double* __restrict__ Ed, const double* _
                            const double* __restrict__ Aud, const double* __restrict__ Aup,
                            const double* __restrict__ pol, double* __restrict__ rd, double* __restrict__ rp,
                            double* __restrict__ zd, double* __restrict__ zp, double* __restrict__ scal,
-                           R4<R>* __restrict__ s4, const int* __restrict__ rank) {
+                           R4<R>* __restrict__ s4, const int* __restrict__ rank, int* __restrict__ done,
+                           int* __restrict__ iter, double thr2, int maxit, cudaGraphConditionalHandle h,
+                           int use_handle, int* __restrict__ cont_out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double rzd = 0, rzp = 0, rrd = 0, rrp = 0;
     if (i < n) {
@@ -104,6 +128,7 @@ __global__ void k_pcg_init(int n, const double* __restrict__ Ed, const double* _
     }
     if (!s4) block_sum_add2(rzd, rzp, scal + RZN_D);
     block_sum_add2(rrd, rrp, scal + RR_D);
+    pcg_decide_last(scal, done, iter, thr2, maxit, 1, h, use_handle, cont_out);
 }
 
 __global__ void k_dot2(int n3, const double* __restrict__ a1, const double* __restrict__ b1,
@@ -158,16 +183,7 @@ __global__ void k_pcg_update(int n, const double* __restrict__ pol, const double
     }
     if (!s4) block_sum_add2(rzd, rzp, scal + RZX_D);
     block_sum_add2(rrd, rrp, scal + RR_D);
-    // the last block to finish (counted in *done, which it resets) takes the
-    // control decision: every block has added its r.r by then
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-            __threadfence();
-            *done = 0;
-            pcg_decide(scal, iter, thr2, maxit, 0, h, use_handle, cont_out);
-        }
-    }
+    pcg_decide_last(scal, done, iter, thr2, maxit, 0, h, use_handle, cont_out);
 }
 
 // beta = rz of this iteration over the last one's (0 on the first iteration)
@@ -249,28 +265,54 @@ __global__ void __launch_bounds__(128) k_pcg_dir_spread(int n, const double* __r
 }
 
 // One preconditioned correction step u += alpha r with the FP64 residual
-// r = E - A u, and the norms of that residual.
+// r = E - A u, and the norms of that residual.  A u is given (Aud, Aup), or
+// (Aud null) assembled here from the real-space fields Fd, Fp and the
+// reciprocal potentials phi as in k_matvec_finish.  With u4 (the forward) also
+// the corrected dipoles' R4 copies in cell order for the force kernels, and
+// with grad their accumulators cleared: one kernel for what took five, each
+// a few microseconds of the evaluation's critical path.
+template <class R>
 __global__ void k_correct(int n, const double* __restrict__ Ed, const double* __restrict__ Ep,
                           const double* __restrict__ Aud, const double* __restrict__ Aup,
-                          const double* __restrict__ pol, double* __restrict__ ud, double* __restrict__ up,
-                          double* __restrict__ resd, double* __restrict__ scal) {
+                          const double* __restrict__ Fd, const double* __restrict__ Fp,
+                          const double* __restrict__ phi, int ewald, double selfc, const double* __restrict__ pol,
+                          double* __restrict__ ud, double* __restrict__ up, double* __restrict__ scal,
+                          R4<R>* __restrict__ u4, const int* __restrict__ rank, double* __restrict__ grad,
+                          double* __restrict__ trq) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double rrd = 0, rrp = 0, urd = 0;
+    double rrd = 0, rrp = 0;
     if (i < n) {
-        double a = pol[i];
+        const double a = pol[i], ia = a > 0 ? 1.0 / a : 0.0;
+        double vd[3], vp[3];
         for (int c = 0; c < 3; c++) {
-            int q = 3 * i + c;
-            double r1 = a > 0 ? Ed[q] - Aud[q] : 0.0, r2 = a > 0 ? Ep[q] - Aup[q] : 0.0;
+            const int q = 3 * i + c;
+            const double d = ud[q], p = up[q];
+            double Ad, Ap;
+            if (Aud) {
+                Ad = Aud[q];
+                Ap = Aup[q];
+            } else {
+                double fd = Fd[q], fp = Fp[q];
+                if (ewald) {
+                    fd += -phi[4 * (size_t)i + 1 + c] + selfc * d;
+                    fp += -phi[4 * ((size_t)n + i) + 1 + c] + selfc * p;
+                }
+                Ad = ia * d - fd;
+                Ap = ia * p - fp;
+            }
+            const double r1 = a > 0 ? Ed[q] - Ad : 0.0, r2 = a > 0 ? Ep[q] - Ap : 0.0;
             rrd += r1 * r1; rrp += r2 * r2;
-            urd += up[q] * r1;   // up . r_d (before the update) for the stationary energy
-            resd[q] = r1;
-            ud[q] += a * r1;
-            up[q] += a * r2;
+            ud[q] = vd[c] = d + a * r1;
+            up[q] = vp[c] = p + a * r2;
+            if (grad) grad[q] = trq[q] = 0;
+        }
+        if (u4) {
+            const int o = rank[i];
+            u4[2 * o] = make_r4<R>((R)vd[0], (R)vd[1], (R)vd[2], R(0));
+            u4[2 * o + 1] = make_r4<R>((R)vp[0], (R)vp[1], (R)vp[2], R(0));
         }
     }
-    block_sum_add(rrd, scal + RR_D);
-    block_sum_add(rrp, scal + RR_P);
-    block_sum_add(urd, scal + RZN_D);
+    block_sum_add2(rrd, rrp, scal + RR_D);
 }
 
 // ep = -1/2 f sum ud . Ep (per-site aep when requested); nep = sites with

@@ -18,7 +18,7 @@ namespace amg {
 // Permanent field at every site from all neighbours' multipoles, bulk
 // (scale 1, Thole damped, Ewald or bare).  Writes Ed = Ep (the d/p
 // differences come only from the scaled pairs).  With COEF the same radial
-// factors also fill the PCG's stored coefficient rows (see k_tu_coeffs: c0 =
+// factors also fill the PCG's stored coefficient rows (see below: c0 =
 // pack_tensor(x_i - x_j, B1, B2)) and the sparse preconditioner's rows (pairs
 // within usolvcut, compacted in row order, when cu0 is given), so the solve's
 // set-up recomputes nothing.
@@ -331,69 +331,6 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 && !VIR && !DDONLY) ? 6 :
 // first matvec, p4, s4) are stored in cell order too: the neighbours of the
 // sites a warp handles then lie in a few contiguous runs of those vectors,
 // which the gathers read as whole cache lines, mostly from L1.
-template <class R, bool EWALD, int LPA, bool CELLS = false>
-__global__ void __launch_bounds__(128) k_tu_coeffs(int n, const int* __restrict__ order, const AtomR<R>* __restrict__ at, Box bx, R aewald,
-                                                   const int* __restrict__ nbr, int cap, const int* __restrict__ nnb,
-                                                   R4<R>* __restrict__ c0, R usolv2, int* __restrict__ nbru,
-                                                   R4<R>* __restrict__ cu0, int* __restrict__ nnbu) {
-    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / LPA, lane = threadIdx.x % LPA;
-    if (g >= n) return;  // whole lane groups leave together
-    const int i = order[g];
-    const int cnt = nnb[i];
-    R4<R> pi = at[g].a, ei = at[g].e;
-    V3<R> xi = v3<R>(pi.x, pi.y, pi.z);
-    const size_t base = (size_t)i * cap;
-    // lanes of this group within the warp, and the lanes below this one
-    const unsigned gmask = LPA == 32 ? 0xffffffffu : ((1u << LPA) - 1u) << ((threadIdx.x & 31) / LPA * LPA);
-    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
-    int nu = 0;  // preconditioner entries of this row so far
-    for (int s0 = 0; s0 < cnt; s0 += LPA) {
-        const int s = s0 + lane;
-        const bool ok = s < cnt;
-        R r2 = 0, P1 = 0, P2 = 0;
-        V3<R> r = v3<R>(0, 0, 0);
-        int j = 0;
-        if (ok) {
-            j = nbr[base + s];
-            R4<R> pj = at[j].a, ej = at[j].e;
-            r = min_image<R, !EWALD || CELLS>(xi - v3<R>(pj.x, pj.y, pj.z), bx);
-            r2 = dot(r, r);
-            R rinv = rsqrt_<R>(r2);
-            R rr = r2 * rinv, rinv2 = rinv * rinv;
-            R b1 = rinv * rinv2, b2 = 3 * b1 * rinv2;
-            R B1 = b1, B2 = b2;
-            if (EWALD) {
-                R eb[3];
-                ewald_terms<R, 3>(rr, rinv2, aewald, eb);
-                B1 = eb[1]; B2 = eb[2];
-            }
-            P1 = b1; P2 = b2;
-            R damp = ei.y * ej.y;
-            if (damp != R(0)) {
-                R t = ratio_<R>(rr, damp);
-                R x = pair_thole<R>(ei.z, ej.z) * t * t * t;
-                R e = exp_<R>(-x);
-                B1 -= e * b1;
-                B2 -= (R(1) + x) * e * b2;
-                P1 -= e * b1;
-                P2 -= (R(1) + x) * e * b2;
-            }
-            c0[base + s] = pack_tensor<R>(r.x, r.y, r.z, B1, B2);
-        }
-        if (cu0) {  // sparse preconditioner: bare Thole-damped T within usolvcut, compacted in order
-            const bool take = ok && r2 <= usolv2;
-            const unsigned b = __ballot_sync(gmask, take) & gmask;
-            if (take) {
-                const size_t q = base + nu + __popc(b & below);
-                nbru[q] = j;
-                cu0[q] = pack_tensor<R>(r.x, r.y, r.z, P1, P2);
-            }
-            nu += __popc(b);
-        }
-    }
-    if (cu0 && lane == 0) nnbu[i] = nu;
-}
-
 // T v with the stored coefficients (both dipole sets): rows of nnb[i] bulk
 // slots plus the site's scaled partners.  u4: [n][2] R4 in cell order.
 // With vAv, also adds -v.F of both sets to vAv[0..1] (the real-space share
@@ -571,7 +508,7 @@ __global__ void k_scaled_coeffs(int np, const ScaledPair* __restrict__ sp, const
 
 // Sparse preconditioner z = M r for both residuals:
 //   z_i = alpha_i (w r_i + sum_j T_ij s_j),  s = alpha r  (packed in s4,
-// cell order), T over the rows built by k_tu_coeffs / k_scaled_coeffs (bulk
+// cell order), T over the rows built by k_perm_field / k_scaled_coeffs (bulk
 // pairs within usolvcut, then the scaled partners; nbru holds the partners'
 // positions in cell order).  Adds r.z of both sets to scal[RZN_D..RZN_P].
 // Blocks stride over the sites (a grid of a few blocks per SM), so each block
