@@ -1316,20 +1316,22 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
             ctx->nbond, ctx->bonds, ctx->bflux, ctx->nangle, ctx->angles, ctx->aflux, ctx->xyz, ctx->dq);
         KCHECK();
     }
-    // neighbour list and real-space permanent field on the side stream (the
-    // list build needs only the positions, so it starts beside the frame
-    // rotations); PME stencils and the reciprocal permanent potential on s
-    cudaStream_t r = fork_side(ctx, s);
-    enqueue_lists(ctx, r);
-    rotate_and_pack<R>(ctx, s);
-    k_zero<double><<<1, 32, 0, s>>>(ctx->status, kStScal);  // accumulators and counters
+    // neighbour list and real-space permanent field on s (the list build needs
+    // only the positions, so it starts beside the frame rotations); the frame
+    // rotations, PME stencils and the reciprocal permanent potential, which
+    // are done long before, on the side stream, whose lower priority leaves
+    // the lists their share of the SMs
+    cudaStream_t m = fork_side(ctx, s);
+    enqueue_lists(ctx, s);
+    rotate_and_pack<R>(ctx, m);
+    k_zero<double><<<1, 32, 0, m>>>(ctx->status, kStScal);  // accumulators and counters
     KCHECK();
-    CK(cudaEventRecord(ctx->erot, s));  // the packed sites for the cell-order copy
-    CK(cudaStreamWaitEvent(r, ctx->erot, 0));
-    k_gather_atoms<R><<<nblk(n), kThreads, 0, r>>>(n, ctx->sids, atoms_of<R>(ctx).at, atoms_of<R>(ctx).atS);
+    CK(cudaEventRecord(ctx->erot, m));  // the packed sites for the cell-order copy
+    CK(cudaStreamWaitEvent(s, ctx->erot, 0));
+    k_gather_atoms<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->sids, atoms_of<R>(ctx).at, atoms_of<R>(ctx).atS);
     KCHECK();
     if (ctx->ewald) {
-        pme_stencils<R>(ctx, s, mixed && iterative(ctx));  // FP64 ones too for the sweep
+        pme_stencils<R>(ctx, m, mixed && iterative(ctx));  // FP64 ones too for the sweep
     }
     CK(cudaEventRecord(ctx->ev[1], s));
     Atoms<R>& A = atoms_of<R>(ctx);
@@ -1340,7 +1342,7 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
         const bool sp = coef && ctx->sparse_prec;
         const R u2 = (R)(ctx->usolvcut * ctx->usolvcut);
         auto launch = [&](auto kern, unsigned nb) {
-            kern<<<nb, kThreads, 0, r>>>(n, ctx->sids, A.atS, ctx->bx, aew, ctx->cnb, ctx->cap, ctx->nnb, ctx->Ed, ctx->Ep,
+            kern<<<nb, kThreads, 0, s>>>(n, ctx->sids, A.atS, ctx->bx, aew, ctx->cnb, ctx->cap, ctx->nnb, ctx->Ed, ctx->Ep,
                                          coef ? A.c0 : nullptr, u2, sp ? ctx->nbru : nullptr,
                                          sp ? A.cu0 : nullptr, sp ? ctx->nnbu : nullptr);
         };
@@ -1358,15 +1360,15 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
             }
         });
         KCHECK();
-        if (coef) build_scaled_coeffs<R>(ctx, r);
+        if (coef) build_scaled_coeffs<R>(ctx, s);
         if (ctx->nsp) {
-            k_scaled_field<<<nblk(ctx->nsp), kThreads, 0, r>>>(ctx->nsp, ctx->sp, ctx->xyz, ctx->rp10, ctx->pdamp,
+            k_scaled_field<<<nblk(ctx->nsp), kThreads, 0, s>>>(ctx->nsp, ctx->sp, ctx->xyz, ctx->rp10, ctx->pdamp,
                                                               ctx->thole, ctx->bx, ctx->cut * ctx->cut, ewald_alpha(ctx),
                                                               ctx->Ed, ctx->Ep);
             KCHECK();
         }
     }
-    if (ctx->ewald) pme_mpole<R>(ctx, s, ctx->want_vir ? ctx->eacc + kVir : nullptr);
+    if (ctx->ewald) pme_mpole<R>(ctx, m, ctx->want_vir ? ctx->eacc + kVir : nullptr);
     join_side(ctx, s);
     if (ctx->has_pol) {
         k_field_finish<R><<<nblk(n), kThreads, 0, s>>>(n, ctx->phiM, ctx->ewald, ctx->rp10, self_coef(ctx), ctx->pol,
