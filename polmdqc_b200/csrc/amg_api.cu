@@ -2123,7 +2123,10 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
         CK(cudaEventCreateWithFlags(&ctx->ejoin[k], cudaEventDisableTiming));
     }
     if (const char* g = getenv("AMG_NO_GRAPH")) ctx->use_graphs = !(g[0] == '1');
-    ctx->lpa = 8;  // lanes per site (8 measured fastest at 12k and 98k sites)
+    // lanes per site of the bulk pair kernels: 8, or 16 where 8 leave the chip
+    // half empty and each lane a long serial share (evaluation with 8 / 16 / 32:
+    // 216 waters 402, 393, 402 us; 1,500: 539, 523, 528; 4,096: 782, 793, 814)
+    ctx->lpa = n <= 8192 ? 16 : 8;
     if (const char* l = getenv("AMG_LPA")) ctx->lpa = atoi(l);
     if (ctx->lpa != 8 && ctx->lpa != 16 && ctx->lpa != 32) ctx->lpa = 16;
     // k_tu_stored uses next to no shared memory, and an SM divided for that
