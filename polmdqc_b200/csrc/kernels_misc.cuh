@@ -332,6 +332,20 @@ __global__ void k_polar_energy(int n, const double* __restrict__ ud, const doubl
     block_sum_add_ll(c, nep);
 }
 
+// sum += g, unless the neighbour lists overflowed (the evaluation is repeated,
+// and the sums go back to the caller as they came)
+__global__ void k_add_gradient(size_t n3, const double* __restrict__ g, const int* __restrict__ overflow, int cap,
+                               double* __restrict__ sum) {
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n3 && *overflow <= cap) sum[q] += g[q];
+}
+
+// *bad = 1 when a value is an infinity or a NaN
+__global__ void k_check_finite(size_t count, const double* __restrict__ x, int* __restrict__ bad) {
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < count && !isfinite(x[q])) *bad = 1;
+}
+
 // ---------------------------------------------------------------- reciprocal
 __device__ __forceinline__ double site_energy(const double* m, const double* p) {
     return m[0] * p[0] + m[1] * p[1] + m[2] * p[2] + m[3] * p[3] + m[4] * p[4] + m[7] * p[5] + m[9] * p[6] +
