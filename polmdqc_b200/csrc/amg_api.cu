@@ -2556,13 +2556,15 @@ int backward_impl(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* gr) 
     const bool opt = ctx->poltyp == AMG_POL_OPT && ctx->npolar > 0;
     const int K = ctx->optorder;
     if (opt && !ctx->adj_opt) dalloc(ctx, ctx->adj_opt, (size_t)(2 * K + 4) * n3);
-    // FP64 copies of the sites (also in cell order), stencils and T coefficients
-    rotate_and_pack<double>(ctx, s);
-    k_gather_atoms<double><<<nblk(n), kThreads, 0, s>>>(n, ctx->sids, ctx->ad.at, ctx->ad.atS);
-    KCHECK();
-    if (ctx->ewald) {
-        pme_prepare<double>(ctx, pme_of<double>(ctx));
-        pme_stencils<double>(ctx, s);
+    // The forward's sites, stencils, rows and permanent potentials are those of
+    // the current coordinates.  What it did not need: in a mixed context the
+    // OPT orders of the cotangents apply the field in FP64.
+    if (opt && ctx->prec == AMG_PREC_MIXED) {
+        rotate_and_pack<double>(ctx, s);
+        if (ctx->ewald) {
+            pme_prepare<double>(ctx, pme_of<double>(ctx));
+            pme_stencils<double>(ctx, s);
+        }
     }
     k_zero<double><<<nblk(2 * n3, 256), 256, 0, s>>>(wd, 2 * n3);
     KCHECK();
@@ -2647,12 +2649,16 @@ int backward_impl(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* gr) 
         if (mixed) pme_dipoles<float, 20>(ctx, s, a, b, ph);
         else pme_dipoles<double, 20>(ctx, s, a, b, ph);
     };
+    // pair kernels on the side stream, the PME of the dipole sets beside them
+    // (they add to the same arrays with atomics or alone; the reciprocal part
+    // follows the join)
+    cudaStream_t r = ctx->ewald ? fork_side(ctx, s) : s;
     if (mixed)
-        adjoint_pairs<float>(ctx, s, vbar, bd, ctx->ud, mwp, ctx->up, mutual, cf, grad, trq, dpd, dth);
+        adjoint_pairs<float>(ctx, r, vbar, bd, ctx->ud, mwp, ctx->up, mutual, cf, grad, trq, dpd, dth);
     else
-        adjoint_pairs<double>(ctx, s, vbar, bd, ctx->ud, mwp, ctx->up, mutual, cf, grad, trq, dpd, dth);
+        adjoint_pairs<double>(ctx, r, vbar, bd, ctx->ud, mwp, ctx->up, mutual, cf, grad, trq, dpd, dth);
     if (ctx->nsp) {
-        k_adjoint_scaled<<<nblk(ctx->nsp), kThreads, 0, s>>>(ctx->nsp, ctx->sp, ctx->xyz, ctx->rp10, ctx->pdamp,
+        k_adjoint_scaled<<<nblk(ctx->nsp), kThreads, 0, r>>>(ctx->nsp, ctx->sp, ctx->xyz, ctx->rp10, ctx->pdamp,
                                                             ctx->thole, ctx->bx, ctx->cut * ctx->cut, ewald_alpha(ctx),
                                                             bd, bp, bd, ctx->ud, mwp, ctx->up, mutual, cf, grad, trq,
                                                             ctx->adj_pot, dpd, dth);
@@ -2660,15 +2666,12 @@ int backward_impl(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* gr) 
     }
     double qtot = 0;
     if (ctx->ewald) {
-        // permanent potentials (overwrite the forward's phiM), in the forward's
-        // grid precision like the dipole potentials below
-        if (mixed) pme_mpole<float>(ctx, s);
-        else pme_mpole<double>(ctx, s);
         double* ph = ctx->adj_phi;
         const size_t blk = 2 * 20 * (size_t)n;
         adj_pme(vbar, bd, ph);              // phi of vbar, P1
         adj_pme(ctx->ud, ctx->up, ph + blk);  // phi of Q1, Q2
         adj_pme(mwp, zeros, ph + 2 * blk);    // phi of P2
+        join_side(ctx, s);
         const size_t one = 20 * (size_t)n;
         k_adjoint_recip<<<nblk(n), kThreads, 0, s>>>(n, ctx->rp10, ctx->phiM, ph, ph + one, ph + blk, ph + 2 * blk,
                                                      ph + blk + one, vbar, bd, ctx->ud, mwp, ctx->up, mutual,
