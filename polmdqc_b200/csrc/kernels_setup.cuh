@@ -141,35 +141,36 @@ __device__ __forceinline__ void frac_wrapped(const CellGrid& cg, double x, doubl
     }
 }
 
+// cell index of a position
+__device__ __forceinline__ unsigned cell_of(const CellGrid& cg, const Box& bx, double x, double y, double z) {
+    int c[3];
+    const double xs[3] = {x, y, z};
+    double f[3];
+    if (cg.general) frac_wrapped(cg, x, y, z, f);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        if (cg.general) {
+            c[a] = min(cg.nc[a] - 1, (int)(f[a] * cg.nc[a]));
+        } else if (cg.centred) {  // wrapped into the enclosing prism
+            f[a] = xs[a] / (cg.size[a] * cg.nc[a]);
+            f[a] -= floor(f[a]);
+            c[a] = min(cg.nc[a] - 1, (int)(f[a] * cg.nc[a]));
+        } else if (cg.periodic) {
+            f[a] = xs[a] * bx.iL[a];
+            f[a] -= floor(f[a]);
+            c[a] = min(cg.nc[a] - 1, (int)(f[a] * cg.nc[a]));
+        } else {
+            c[a] = min(cg.nc[a] - 1, max(0, (int)((xs[a] - cg.origin[a]) / cg.size[a])));
+        }
+    }
+    return (unsigned)((c[0] * cg.nc[1] + c[1]) * cg.nc[2] + c[2]);
+}
+
 __global__ void k_cell_index(int n, const double* __restrict__ xyz, CellGrid cg, Box bx, unsigned* __restrict__ keys,
                              int* __restrict__ ids) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int c[3];
-    if (cg.general) {
-        double f[3];
-        frac_wrapped(cg, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], f);
-        for (int a = 0; a < 3; a++) c[a] = min(cg.nc[a] - 1, (int)(f[a] * cg.nc[a]));
-        keys[i] = (unsigned)((c[0] * cg.nc[1] + c[1]) * cg.nc[2] + c[2]);
-        ids[i] = i;
-        return;
-    }
-    for (int a = 0; a < 3; a++) {
-        double x = xyz[3 * i + a];
-        double f;
-        if (cg.centred) {  // wrapped into the enclosing prism
-            f = x / (cg.size[a] * cg.nc[a]);
-            f -= floor(f);
-            c[a] = min(cg.nc[a] - 1, (int)(f * cg.nc[a]));
-        } else if (cg.periodic) {
-            f = x * bx.iL[a];
-            f -= floor(f);
-            c[a] = min(cg.nc[a] - 1, (int)(f * cg.nc[a]));
-        } else {
-            c[a] = min(cg.nc[a] - 1, max(0, (int)((x - cg.origin[a]) / cg.size[a])));
-        }
-    }
-    keys[i] = (unsigned)((c[0] * cg.nc[1] + c[1]) * cg.nc[2] + c[2]);
+    keys[i] = cell_of(cg, bx, xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]);
     ids[i] = i;
 }
 

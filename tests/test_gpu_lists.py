@@ -1,7 +1,8 @@
 """The cell-grid neighbour lists at the edges of their staging: fewer and more
 hits than a warp's queue holds, more home sites and candidates than one chunk,
-a last chunk that is not a multiple of the scan, two blocks per cell, and sites
-with more scaled partners than a warp has lanes.  The pair count is exact
+a last chunk that is not a multiple of the scan, two blocks per cell, sites
+with more scaled partners than a warp has lanes, and the cell order by counting
+with cells of more and fewer sites than a warp.  The pair count is exact
 against the FP64 oracle; energies and gradients at the FP64 path's tolerances
 against it (the same pairs, FP64 sums in another order)."""
 import dataclasses
@@ -35,6 +36,8 @@ def many_partners(s, count):
     (512, 24.9, 4.0, 0),     # 6 cells per axis
     (1331, 34.2, 11.3, 0),   # ~150 sites per cell, ~4,000 candidates
     (216, 18.643, 6.0, 40),  # rows with more than 32 scaled partners
+    (2197, 40.4, 9.0, 0),    # sites ordered by counting: 64 cells of ~100 sites
+    (2200, 80.0, 5.0, 0),    # ... 4,096 cells, most of 1 or 2 sites
 ])
 def test_lists_match_the_oracle(waters, box, cutoff, partners):
     s = systems.water_box(waters, box, seed=waters)
