@@ -2,9 +2,10 @@
 // include/amoeba_gpu.h, device buffers, cuFFT plans and the evaluation
 // pipeline (frames -> lists -> permanent field -> PCG -> energies/forces).
 //
-// One context = one device, one stream.  Everything between amg_set_coords
-// and the result copy stays on the device; the PCG convergence test reads
-// two FP64 scalars per iteration.
+// One context = one device and a handful of streams of its own, forked from
+// and joined to one.  Everything between amg_set_coords and the result copy
+// stays on the device; in a captured evaluation the PCG's last kernel decides
+// there whether the loop goes on.
 #include "../../include/amoeba_gpu.h"
 #include "kernels_setup.cuh"
 #include "kernels_pme.cuh"

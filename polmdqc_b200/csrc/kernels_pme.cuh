@@ -6,8 +6,9 @@
 // sets are spread into one complex grid g = Q_d + i Q_p: the influence
 // function G is real and even (G(m) = G(-m)), so
 //   IFFT(G . FFT(Q_d + i Q_p)) = (G * Q_d) + i (G * Q_p)
-// and one in-place complex transform pair (library C2C, unnormalised both
-// ways as in smooth PME) convolves both sets.
+// and one complex transform pair, unnormalised both ways as in smooth PME,
+// convolves both sets (kernels_fft.cuh; the library's C2C for sizes that are no
+// product of two small radices and where the virial needs the transform).
 #pragma once
 #include "kernels.cuh"
 #include "kernels_setup.cuh"
