@@ -1147,7 +1147,7 @@ void build_scaled_coeffs(amg_ctx* ctx, cudaStream_t s) {
     KCHECK();
 }
 
-// Blocks of k_tu_stored per SM.  In FP32 9 blocks fit an SM (54 registers),
+// Blocks of k_tu_stored per SM.  In FP32 9 blocks fit an SM (56 registers),
 // and a grid that fills them all leaves no room for the PME chain's blocks
 // beside it until its last wave: with 6 striding blocks the chain runs
 // through (32,768 waters: 3.67 -> 3.54 ms per evaluation; 4 blocks 3.58, 8
