@@ -15,6 +15,7 @@
 #include "kernels_adjoint.cuh"
 #include "kernels_cp.cuh"
 #include "kernels_order.cuh"
+#include "graph_slot.h"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cufft.h>
@@ -1709,6 +1710,20 @@ cudaError_t install_graph(cudaGraphExec_t& exec, cudaGraph_t graph) {
     return e;
 }
 
+// ends and discards captures that are under way: the loop body's on st2, the
+// evaluation's (which owns the body) on st
+void abandon(amg_ctx* ctx) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t g = nullptr;
+    if (cudaStreamIsCapturing(ctx->st2, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone)
+        cudaStreamEndCapture(ctx->st2, &g);
+    g = nullptr;
+    if (cudaStreamIsCapturing(ctx->st, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone)
+        cudaStreamEndCapture(ctx->st, &g);
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+}
+
 // Captures the whole evaluation as one CUDA graph: the PCG loop is a
 // conditional WHILE node whose body is one iteration; its last kernel sets
 // the condition from the FP64 residual norms on the device.
@@ -1716,20 +1731,15 @@ template <class R>
 bool capture_graph(amg_ctx* ctx, int flags) {
     cudaStream_t s = ctx->st;
     cudaGraph_t graph = nullptr;
+    const long long k0 = ctx->kcount;
     auto fail = [&](const char* what, cudaError_t e) {
         ctx->graph_note = std::string(what) + ": " + cudaGetErrorString(e);
-        cudaStreamCaptureStatus st;
-        if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) {
-            cudaGraph_t g2;
-            cudaStreamEndCapture(s, &g2);
-            if (g2) cudaGraphDestroy(g2);
-        }
-        cudaGetLastError();
+        abandon(ctx);
+        ctx->kcount = k0;
         return false;
     };
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail("begin capture", e);
-    const long long k0 = ctx->kcount;
     long long kb = 0;
     try {
         enqueue_front<R>(ctx, s);
@@ -1868,13 +1878,12 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
         bool graphed = false;
         const long long kstart = ctx->kcount;
         if (ctx->use_graphs && ctx->bounds) {
-            if (ctx->graph_dirty || !ctx->gexec || ctx->gflags != flags) capture_graph<R>(ctx, flags);
-            if (ctx->gexec) {
-                CK(cudaGraphLaunch(ctx->gexec, st));
-                graphed = true;
-            }
+            graphed = launchable(ctx->gexec, ctx->graph_dirty || ctx->gflags != flags,
+                                 [&] { return capture_graph<R>(ctx, flags); }, cudaGraphExecDestroy);
+            if (graphed) CK(cudaGraphLaunch(ctx->gexec, st));
         }
         if (!graphed) enqueue_eager<R>(ctx, flags);
+        ctx->graphed_last = graphed;
         ctx->klast = graphed ? -1 : ctx->kcount - kstart;  // graph: completed below from the iteration count
         // status and gradients behind one synchronisation.  The gradients come
         // in pieces, each with its event: the host adds a piece to the
@@ -1980,7 +1989,6 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
         // history: start the history again
         if (ctx->pred_state) CK(cudaMemsetAsync(ctx->pred_state, 0, 2 * sizeof(int), st));
     }
-    ctx->graphed_last = ctx->use_graphs && ctx->bounds && ctx->gexec != nullptr;
     // ---- results
     const double* e = ctx->rb;
     const double* hs = ctx->rb + kStScal;
@@ -2479,13 +2487,7 @@ bool capture_adjoint(amg_ctx* ctx) {
     cudaGraph_t graph = nullptr;
     const long long k0 = ctx->kcount;
     auto fail = [&](cudaError_t) {
-        cudaStreamCaptureStatus st;
-        if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) {
-            cudaGraph_t g2 = nullptr;
-            cudaStreamEndCapture(s, &g2);
-            if (g2) cudaGraphDestroy(g2);
-        }
-        cudaGetLastError();
+        abandon(ctx);
         ctx->kcount = k0;
         return false;
     };
@@ -2542,8 +2544,8 @@ void adjoint_solve(amg_ctx* ctx, cudaStream_t s) {
     // (captured with the vectors the caller set; they are the same buffers on
     // every call)
     if (ctx->use_graphs && ctx->bounds && ctx->gexec) {
-        if (!ctx->adj_gexec || ctx->adj_gen != ctx->fwd_gen) capture_adjoint<R>(ctx);
-        if (ctx->adj_gexec) {
+        if (launchable(ctx->adj_gexec, ctx->adj_gen != ctx->fwd_gen, [&] { return capture_adjoint<R>(ctx); },
+                       cudaGraphExecDestroy)) {
             CK(cudaGraphLaunch(ctx->adj_gexec, s));
             return;
         }
