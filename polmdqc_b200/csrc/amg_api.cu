@@ -236,6 +236,8 @@ struct amg_ctx {
     int* rb_over_m = nullptr;       // pinned: the overflow flag read with the permanent-multipole gradient
     double* gsum = nullptr;         // [2][3n] the caller's gradient arrays on their way through the device
     cudaEvent_t gsum_in = nullptr;  // their old values are there
+    double* xyz_stage = nullptr;    // pinned [3n]: coordinates on their way (below kGpuHostArrays values)
+    cudaEvent_t xyz_in = nullptr;   // they have left it
     int* h_bad = nullptr;           // pinned: the coordinate check's answer
     std::vector<double> rb_pole;    // [10n] rotated multipoles on their way to amg_results.rpole
     cudaEvent_t rbev[1 + kRbChunks] = {};  // scalars read back, then each gradient piece
@@ -2078,6 +2080,8 @@ void release(amg_ctx* ctx) {
     if (ctx->rb_over_m) { cudaFreeHost(ctx->rb_over_m); ctx->rb_over_m = nullptr; }
     if (ctx->h_bad) { cudaFreeHost(ctx->h_bad); ctx->h_bad = nullptr; }
     if (ctx->gsum_in) { cudaEventDestroy(ctx->gsum_in); ctx->gsum_in = nullptr; }
+    if (ctx->xyz_stage) { cudaFreeHost(ctx->xyz_stage); ctx->xyz_stage = nullptr; }
+    if (ctx->xyz_in) { cudaEventDestroy(ctx->xyz_in); ctx->xyz_in = nullptr; }
     dfree(ctx->gsum);
     for (auto& e : ctx->rbev)
         if (e) { cudaEventDestroy(e); e = nullptr; }
@@ -2251,6 +2255,7 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     for (auto& e : ctx->ev) CK(cudaEventCreate(&e));
     CK(cudaEventCreateWithFlags(&ctx->erot, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ctx->gm_ready, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ctx->xyz_in, cudaEventDisableTiming));
     CK(cudaStreamCreateWithFlags(&ctx->rbst, cudaStreamNonBlocking));
     upload(ctx, ctx->pole13, P->pole, 13 * (size_t)n);
     upload(ctx, ctx->zax, P->zaxis, n);
@@ -2867,9 +2872,22 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
         ctx->have_coords = false;
         ctx->have_forward = false;
         const size_t n3 = 3 * (size_t)ctx->n;
-        CK(cudaMemcpyAsync(ctx->xyz, xyz, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
+        // The array is the caller's again when the call returns.  A copy from
+        // pinned memory is read by the device in its own time, so small arrays
+        // go through pinned memory of the context (waiting for the device here
+        // instead costs its latency, which the launch that follows hides: 216
+        // waters 390 -> 402 us per step); large ones are waited for.
         bool finite;
-        if (gpu_handles(xyz, n3)) {
+        if (n3 < kGpuHostArrays) {
+            if (!ctx->xyz_stage) CK(cudaMallocHost((void**)&ctx->xyz_stage, sizeof(double) * n3));
+            CK(cudaEventSynchronize(ctx->xyz_in));
+            std::memcpy(ctx->xyz_stage, xyz, sizeof(double) * n3);
+            CK(cudaMemcpyAsync(ctx->xyz, ctx->xyz_stage, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
+            CK(cudaEventRecord(ctx->xyz_in, ctx->st));
+            xyz = ctx->xyz_stage;
+            finite = all_finite(xyz, n3);
+        } else if (gpu_handles(xyz, n3)) {
+            CK(cudaMemcpyAsync(ctx->xyz, xyz, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
             if (!ctx->h_bad) CK(cudaMallocHost((void**)&ctx->h_bad, sizeof(int)));
             int* bad = ctx->iter + 2;  // in the status block
             CK(cudaMemsetAsync(bad, 0, sizeof(int), ctx->st));
@@ -2879,7 +2897,9 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
             CK(cudaStreamSynchronize(ctx->st));
             finite = !*ctx->h_bad;
         } else {
+            CK(cudaMemcpyAsync(ctx->xyz, xyz, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
             finite = all_finite(xyz, n3);
+            CK(cudaStreamSynchronize(ctx->st));
         }
         if (!finite) {
             ctx->err = "non-finite coordinate";
@@ -2888,6 +2908,8 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
         cell_grid(ctx, xyz);
         ctx->have_coords = true;
     } catch (Fail& f) {
+        cudaStreamSynchronize(ctx->st);
+        cudaGetLastError();
         return f.code;
     }
     return AMG_OK;
