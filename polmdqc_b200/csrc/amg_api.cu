@@ -1201,12 +1201,6 @@ void matvec_stored(amg_ctx* ctx, cudaStream_t s, const R4<R>* v4, const double* 
 }
 
 bool iterative(const amg_ctx* ctx) { return ctx->has_pol && ctx->poltyp == AMG_POL_MUTUAL && ctx->npolar > 0; }
-// models that apply the dipole field several times store its coefficient rows
-// once (OPT4, 6,859 waters: four orders of 42 us on the fly against one pass of
-// 24 us more and four of 15: 921 -> 850 us per evaluation)
-bool stored_rows(const amg_ctx* ctx) {
-    return iterative(ctx) || (ctx->has_pol && ctx->poltyp == AMG_POL_OPT && ctx->npolar > 0);
-}
 
 double pcg_threshold(const amg_ctx* ctx) {
     double t = ctx->poleps / ctx->debye;
@@ -1379,8 +1373,8 @@ void enqueue_front(amg_ctx* ctx, cudaStream_t s) {
     Atoms<R>& A = atoms_of<R>(ctx);
     const R aew = (R)ctx->aewald;
     if (ctx->has_pol) {
-        // with a solve (or OPT orders) to follow, the same pass fills the coefficient rows
-        const bool coef = stored_rows(ctx);
+        // with a solve to follow, the same pass fills the PCG's coefficient rows
+        const bool coef = iterative(ctx);
         const bool sp = coef && ctx->sparse_prec;
         const R u2 = (R)(ctx->usolvcut * ctx->usolvcut);
         auto launch = [&](auto kern, unsigned nb) {
@@ -1434,9 +1428,7 @@ void enqueue_opt(amg_ctx* ctx, cudaStream_t s) {
     KCHECK();
     for (int k = 1; k <= ctx->optorder; k++) {
         const double* vd = uo + (k - 1) * blk;
-        k_pack_u<R><<<nblk(ctx->n), kThreads, 0, s>>>(ctx->n, vd, vd + n3, atoms_of<R>(ctx).u4, ctx->rank);
-        KCHECK();
-        matvec_stored<R>(ctx, s, atoms_of<R>(ctx).u4, vd, vd + n3, ctx->Apd, ctx->App);
+        matvec<R>(ctx, s, vd, vd + n3, ctx->Apd, ctx->App);
         k_opt_step<<<nblk(n3), kThreads, 0, s>>>(n3, ctx->pol, vd, vd + n3, ctx->Apd, ctx->App, ctx->copm.c[k],
                                                  uo + k * blk, uo + k * blk + n3, ctx->ud, ctx->up);
         KCHECK();
@@ -1872,7 +1864,7 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     double* gm = ctx->rb + kStatus + n3;
     for (int attempt = 0; attempt < 2; attempt++) {
         ensure_list_buffers(ctx);
-        if (stored_rows(ctx)) ensure_coeff_buffers<R>(ctx, atoms_of<R>(ctx));
+        if (iterative(ctx)) ensure_coeff_buffers<R>(ctx, atoms_of<R>(ctx));
         if (ctx->ewald) {
             pme_prepare<R>(ctx, pme_of<R>(ctx));
             if (ctx->prec == AMG_PREC_MIXED && iterative(ctx)) pme_prepare<double>(ctx, pme_of<double>(ctx));
