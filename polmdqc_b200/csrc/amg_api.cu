@@ -236,8 +236,9 @@ struct amg_ctx {
     int* rb_over_m = nullptr;       // pinned: the overflow flag read with the permanent-multipole gradient
     double* gsum = nullptr;         // [2][3n] the caller's gradient arrays on their way through the device
     cudaEvent_t gsum_in = nullptr;  // their old values are there
-    double* xyz_stage = nullptr;    // pinned [3n]: coordinates on their way (below kGpuHostArrays values)
-    cudaEvent_t xyz_in = nullptr;   // they have left it
+    double* xyz_stage = nullptr;    // pinned [3n]: coordinates on their way (up to kStageCoords values)
+    bool xyz_moving = false;        // they may not have left it yet
+    cudaEvent_t xyz_in = nullptr;   // the caller's coordinates are on the device (more values)
     int* h_bad = nullptr;           // pinned: the coordinate check's answer
     std::vector<double> rb_pole;    // [10n] rotated multipoles on their way to amg_results.rpole
     cudaEvent_t rbev[1 + kRbChunks] = {};  // scalars read back, then each gradient piece
@@ -2059,6 +2060,7 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     ctx->timing[0] = ms[0] + ms[1] + ms[2] + ms[3];
     for (int k = 0; k < 4; k++) ctx->timing[k + 1] = ms[k];
     ctx->have_forward = true;
+    ctx->xyz_moving = false;
     if (!std::isfinite(res->em) || !std::isfinite(res->ep)) {
         ctx->err = "non-finite energy";
         return AMG_ERR_NAN;
@@ -2864,18 +2866,21 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
         ctx->have_coords = false;
         ctx->have_forward = false;
         const size_t n3 = 3 * (size_t)ctx->n;
-        // The array is the caller's again when the call returns.  A copy from
-        // pinned memory is read by the device in its own time, so small arrays
-        // go through pinned memory of the context (waiting for the device here
-        // instead costs its latency, which the launch that follows hides: 216
-        // waters 390 -> 402 us per step); large ones are waited for.
-        bool finite;
-        if (n3 < kGpuHostArrays) {
+        // The array is the caller's again when the call returns, but a copy from
+        // pinned memory is read by the device in its own time.  So up to
+        // kStageCoords values go through pinned memory of the context; more are
+        // waited for at the end, when the device has them, as a rule (step with
+        // three contexts taking turns, unwaited / staged / waited for: 648 sites
+        // 403 / 403 / 414 us, 4,500: 580 / 580 / 591, 12,288: 853 / 866 / 857,
+        // 24,044 in FP64 1,889 / 1,925 / 1,895).
+        constexpr size_t kStageCoords = 16384;
+        bool finite, wait = false;
+        if (n3 <= kStageCoords) {
             if (!ctx->xyz_stage) CK(cudaMallocHost((void**)&ctx->xyz_stage, sizeof(double) * n3));
-            CK(cudaEventSynchronize(ctx->xyz_in));
+            if (ctx->xyz_moving) CK(cudaStreamSynchronize(ctx->st));
             std::memcpy(ctx->xyz_stage, xyz, sizeof(double) * n3);
             CK(cudaMemcpyAsync(ctx->xyz, ctx->xyz_stage, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
-            CK(cudaEventRecord(ctx->xyz_in, ctx->st));
+            ctx->xyz_moving = true;
             xyz = ctx->xyz_stage;
             finite = all_finite(xyz, n3);
         } else if (gpu_handles(xyz, n3)) {
@@ -2890,14 +2895,19 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
             finite = !*ctx->h_bad;
         } else {
             CK(cudaMemcpyAsync(ctx->xyz, xyz, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
+            CK(cudaEventRecord(ctx->xyz_in, ctx->st));
             finite = all_finite(xyz, n3);
-            CK(cudaStreamSynchronize(ctx->st));
+            wait = true;
+        }
+        if (finite) cell_grid(ctx, xyz);
+        if (wait && cudaEventQuery(ctx->xyz_in) != cudaSuccess) {
+            cudaGetLastError();  // "not ready" is no error
+            CK(cudaEventSynchronize(ctx->xyz_in));
         }
         if (!finite) {
             ctx->err = "non-finite coordinate";
             return AMG_ERR_NAN;
         }
-        cell_grid(ctx, xyz);
         ctx->have_coords = true;
     } catch (Fail& f) {
         cudaStreamSynchronize(ctx->st);

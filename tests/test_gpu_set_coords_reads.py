@@ -19,7 +19,8 @@ def pinned(a):
     return torch.from_numpy(np.array(a, np.float64).reshape(-1)).pin_memory().numpy()
 
 
-@pytest.mark.parametrize("waters, box, nfft", [(216, 18.643, 24), (11000, 69.1, 72)])  # below and above the GPU's share
+@pytest.mark.parametrize("waters, box, nfft", [(216, 18.643, 24), (1820, 37.9, 40), (1821, 37.9, 40), (2744, 43.5, 48),
+                                               (11000, 69.1, 72)])  # staged (up to 16,384 values), waited for, the GPU's
 def test_coordinates_are_read_before_the_call_returns(waters, box, nfft):
     s = systems.water_box(waters, box, seed=5)
     other = systems.water_box(waters, box, seed=6).xyz.reshape(-1)
@@ -47,6 +48,15 @@ def test_coordinates_are_read_before_the_call_returns(waters, box, nfft):
             e.set_coords(xyz)
         xyz[:] = other
         e.set_coords(s.xyz)
+        assert abs(e.forward(FLAGS).em - ref.em) <= 1e-9 * abs(ref.em)
+        # two calls in a row: the second one's coordinates
+        xyz[:] = other
+        with torch.cuda.stream(side):
+            dst.copy_(big, non_blocking=True)
+        e.set_coords(xyz)
+        xyz[:] = s.xyz.reshape(-1)
+        e.set_coords(xyz)
+        xyz[:] = other
         assert abs(e.forward(FLAGS).em - ref.em) <= 1e-9 * abs(ref.em)
     finally:
         torch.cuda.synchronize()
