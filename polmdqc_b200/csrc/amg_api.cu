@@ -18,6 +18,7 @@
 #include "graph_slot.h"
 
 #include <cub/device/device_radix_sort.cuh>
+#include <cuda.h>
 #include <cufft.h>
 
 #include <algorithm>
@@ -1816,18 +1817,44 @@ void enqueue_eager(amg_ctx* ctx, int flags) {
     enqueue_back<R>(ctx, s, flags);
 }
 
-// whether the GPU is to handle a caller's array itself: large, and pinned (at
-// both ends; copies of it are the driver's own, which takes any memory)
-bool gpu_handles(const double* p, size_t count) {
-    if (!p || count < kGpuHostArrays) return false;
-    for (const double* q : {p, p + count - 1}) {
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, q) != cudaSuccess || at.type != cudaMemoryTypeHost) {
+// [start, end) of the one pinned allocation or registration that holds p (the
+// driver's own pointer query: the runtime's tells a kind but no extent); false
+// where there is none
+bool pinned_range(const void* p, uintptr_t& start, uintptr_t& end) {
+    using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return false;
+            f = nullptr;
         }
+        return reinterpret_cast<Query>(f);
+    }();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeHost) {
+        cudaGetLastError();
+        return false;
     }
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (!query ||
+        query(&base, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS)
+        return false;
+    start = (uintptr_t)base;
+    end = start + size;
     return true;
+}
+
+// whether the GPU is to handle a caller's array itself: large, and all of it in
+// one pinned range (an array may span several registrations, or only begin and
+// end in them: a copy of that is refused, and the host takes any memory)
+bool gpu_handles(const double* p, size_t count) {
+    uintptr_t start, end;
+    if (!p || count < kGpuHostArrays || !pinned_range(p, start, end)) return false;
+    return (uintptr_t)p >= start && (uintptr_t)(p + count) <= end;
 }
 
 // Touches every page of a caller's output array (writes back what is there)
