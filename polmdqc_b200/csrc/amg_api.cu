@@ -330,6 +330,11 @@ void upload(amg_ctx* ctx, T*& d, const T* h, size_t count) {
     if (h && count) CK(cudaMemcpy(d, h, sizeof(T) * count, cudaMemcpyHostToDevice));
 }
 
+// Set-up clears and uploads on the legacy stream, and a small upload from
+// pageable memory may return with its last part on the way: the context's own
+// streams, which are not ordered after that stream, start behind this.
+void finish_setup(amg_ctx* ctx) { CK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 // ------------------------------------------------------------ scaled pairs
 // The scaled-pair table: m-scales by 1-2..1-5 (applied in order, a later
 // list overwrites, as the reference's exclusion set-up at
@@ -572,6 +577,7 @@ void pme_prepare(amg_ctx* ctx, Pme<R>& pm) {
         }
         upload(ctx, pm.bsmod, mod.data(), mod.size());
         fft_prepare(ctx, pm);
+        finish_setup(ctx);
         pm.ready = true;
     }
     if (!std::equal(ctx->box, ctx->box + 6, pm.infl_box)) {
@@ -814,7 +820,7 @@ void ensure_coeff_buffers(amg_ctx* ctx, Atoms<R>& A) {
         dalloc(ctx, A.cu0, (size_t)ctx->cap * ctx->n);
         if (!A.s4) {
             dalloc(ctx, A.s4, 2 * (size_t)ctx->n);
-            CK(cudaMemset(A.s4, 0, sizeof(R4<R>) * 2 * (size_t)ctx->n));  // the w words stay zero
+            CK(cudaMemsetAsync(A.s4, 0, sizeof(R4<R>) * 2 * (size_t)ctx->n, ctx->st));  // the w words stay zero
         }
     }
     A.cap = ctx->cap;
@@ -2821,6 +2827,7 @@ int amg_create(const amg_params* params, amg_ctx** out) {
     amg_ctx* ctx = new amg_ctx();
     try {
         rc = create_impl(ctx, params);
+        finish_setup(ctx);
     } catch (Fail& f) {
         rc = f.code;
     }
