@@ -2102,6 +2102,29 @@ int forward_impl(amg_ctx* ctx, int flags, amg_results* res) {
     return status;
 }
 
+// After a call that failed between its kernels: nothing of it runs on, no copy
+// to or from the caller's arrays outlives it, and what an evaluation takes for
+// clear (the PME grids and the cells' counts between their uses, the last-block
+// counter) is clear for the next call; a backward needs a new forward.
+void recover(amg_ctx* ctx) {
+    ctx->have_forward = false;
+    for (cudaStream_t s : {ctx->st, ctx->st2, ctx->side[0], ctx->side[1], ctx->side[2], ctx->rbst})
+        if (s) cudaStreamSynchronize(s);
+    auto clear = [&](void* p, size_t bytes) {
+        if (p) cudaMemsetAsync(p, 0, bytes, ctx->st);
+    };
+    auto grids = [&](auto& pm) {
+        if (!pm.ready) return;
+        clear(pm.grid, sizeof(*pm.grid) * pm.G);
+        clear(pm.zg, sizeof(*pm.zg) * pm.G);
+    };
+    grids(pme_of<float>(ctx));
+    grids(pme_of<double>(ctx));
+    clear(ctx->ccount, sizeof(int) * ctx->ncell_alloc);
+    clear(ctx->blk_done, sizeof(int));
+    cudaGetLastError();
+}
+
 void release(amg_ctx* ctx) {
     if (ctx->rb) { cudaFreeHost(ctx->rb); ctx->rb = nullptr; }
     if (ctx->rb_over_m) { cudaFreeHost(ctx->rb_over_m); ctx->rb_over_m = nullptr; }
@@ -2944,8 +2967,7 @@ int amg_set_coords(amg_ctx* ctx, const double* xyz, const double box[6]) {
         }
         ctx->have_coords = true;
     } catch (Fail& f) {
-        cudaStreamSynchronize(ctx->st);
-        cudaGetLastError();
+        recover(ctx);
         return f.code;
     }
     return AMG_OK;
@@ -2963,10 +2985,7 @@ int amg_forward(amg_ctx* ctx, int32_t flags, amg_results* res) {
         if (ctx->prec == AMG_PREC_MIXED) return forward_impl<float>(ctx, flags, res);
         return forward_impl<double>(ctx, flags, res);
     } catch (Fail& f) {
-        // no copy to or from the caller's arrays outlives the call
-        cudaStreamSynchronize(ctx->rbst);
-        cudaStreamSynchronize(ctx->st);
-        cudaGetLastError();
+        recover(ctx);
         return f.code;
     }
 }
@@ -2981,6 +3000,7 @@ int amg_backward(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* grads
         CK(cudaSetDevice(ctx->device));
         return backward_impl(ctx, cot, grads);
     } catch (Fail& f) {
+        recover(ctx);
         return f.code;
     }
 }
@@ -3042,6 +3062,7 @@ int amg_bench(amg_ctx* ctx, int32_t flags, int32_t steps, int64_t flush_bytes, d
             return AMG_ERR_CUDA;
         }
     } catch (Fail& f) {
+        recover(ctx);
         return f.code;
     }
     return AMG_OK;
