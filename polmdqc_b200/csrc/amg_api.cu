@@ -36,7 +36,6 @@ using namespace amg;
 namespace {
 
 constexpr int kOrder = 5;        // B-spline order compiled in (pme.h bseorder default)
-constexpr int kGatherLanes = 4;  // lanes per site in the PME gathers (8: within 3% either way up to 12,288 sites, slower above)
 constexpr int kThreads = 128;
 // Gradient read-back in at most kRbChunks pieces of at least kRbPiece values:
 // a copy costs a few microseconds whatever its size
@@ -1016,7 +1015,7 @@ void pme_mpole(amg_ctx* ctx, cudaStream_t s, double* vir = nullptr) {
     k_convolve<R><<<nblk(pm.Gc, 256), 256, 0, s>>>(pm.Gc, 1, pm.infl, (typename Cplx<R>::type*)pm.cgrid, pm.grid, pm.G);
     KCHECK();
     CKFFT(CufftTypes<R>::inv(pm.i1, pm.cgrid, pm.phig));
-    k_gather<R, kOrder, 20, kGatherLanes, 1><<<nblk((size_t)ctx->n * kGatherLanes), kThreads, 0, s>>>(
+    k_gather<R, kOrder, 20, 1><<<nblk((size_t)ctx->n * kLineLanes), kThreads, 0, s>>>(
         ctx->n, pm.phig, pm.theta, pm.k0, K, ctx->frac, ctx->phiM);
     KCHECK();
 }
@@ -1024,9 +1023,10 @@ void pme_mpole(amg_ctx* ctx, cudaStream_t s, double* vir = nullptr) {
 // spread two dipole sets into the complex grid pm.zg (d + i p), transform,
 // convolve into pm.zq (clearing pm.zg for the next spreading) and transform
 // pm.zq back in place.  `spread` false: the grid already holds the spread
-// dipoles (the PCG's fused direction update put them there).  The PCG's
-// last direction update leaves a spread grid behind, so every other caller
-// clears it first.
+// dipoles (the PCG's fused direction update put them there).  The grid is clear
+// between uses; it is cleared before the spreading all the same, which costs
+// nothing (without: 24,044 sites in FP64 1,854 -> 1,830 us, 12,288 sites 827 ->
+// 830, 20,577 with OPT4 850 -> 860).
 template <class R>
 void spread_dipoles(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp) {
     Pme<R>& pm = pme_of<R>(ctx);
@@ -1040,10 +1040,10 @@ void spread_dipoles(amg_ctx* ctx, cudaStream_t s, const double* vd, const double
 // transform and the permanent one saved by pme_mpole
 template <class R>
 void pme_dipole_grids(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp, bool spread = true,
-                      double* vir = nullptr, bool mterms = true, bool clear = true) {
+                      double* vir = nullptr, bool mterms = true) {
     Pme<R>& pm = pme_of<R>(ctx);
     if (spread) {
-        if (clear) CK(cudaMemsetAsync(pm.zg, 0, sizeof(typename Cplx<R>::type) * pm.G, s));
+        CK(cudaMemsetAsync(pm.zg, 0, sizeof(typename Cplx<R>::type) * pm.G, s));
         spread_dipoles<R>(ctx, s, vd, vp);
     }
     if (pm.own_fft && !vir) {  // the virial needs the transform before the convolution
@@ -1071,7 +1071,7 @@ void pme_dipoles(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* v
     Pme<R>& pm = pme_of<R>(ctx);
     int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
     pme_dipole_grids<R>(ctx, s, vd, vp, true, vir, mterms);
-    k_gather<R, kOrder, NC, kGatherLanes, 2><<<nblk((size_t)ctx->n * kGatherLanes), kThreads, 0, s>>>(
+    k_gather<R, kOrder, NC, 2><<<nblk((size_t)ctx->n * kLineLanes), kThreads, 0, s>>>(
         ctx->n, pm.zq, pm.theta, pm.k0, K, ctx->frac, phi);
     KCHECK();
 }
@@ -1178,7 +1178,7 @@ unsigned tu_blocks(const amg_ctx* ctx, int lanes) {
 // of v.Av, and the caller takes A v = Ad - Fd (k_pcg_update).
 template <class R>
 void matvec_stored(amg_ctx* ctx, cudaStream_t s, const R4<R>* v4, const double* vd, const double* vp, double* Ad,
-                   double* Ap, double* vAv = nullptr, bool spread = true, bool apart = false, bool clear = true) {
+                   double* Ap, double* vAv = nullptr, bool spread = true, bool apart = false) {
     const int n = ctx->n;
     Atoms<R>& A = atoms_of<R>(ctx);
     apart = apart && ctx->ewald && vAv;
@@ -1192,12 +1192,11 @@ void matvec_stored(amg_ctx* ctx, cudaStream_t s, const R4<R>* v4, const double* 
     KCHECK();
     if (ctx->ewald) {
         Pme<R>& pm = pme_of<R>(ctx);
-        pme_dipole_grids<R>(ctx, s, vd, vp, spread, nullptr, true, clear);
+        pme_dipole_grids<R>(ctx, s, vd, vp, spread);
         if (!apart) join_side(ctx, s);
         int3 K = make_int3(ctx->K[0], ctx->K[1], ctx->K[2]);
-        constexpr int G = kGatherLanes;
-        const unsigned blocks = (unsigned)std::min<size_t>(nblk((size_t)n * G), (size_t)ctx->num_sms * 8);
-        k_gather_field<R, kOrder, G><<<blocks, kThreads, 0, s>>>(n, pm.zq, pm.rec, K, ctx->frac, vd, vp, apart ? nullptr : ctx->Fd,
+        const unsigned blocks = (unsigned)std::min<size_t>(nblk((size_t)n * kLineLanes), (size_t)ctx->num_sms * 8);
+        k_gather_field<R, kOrder><<<blocks, kThreads, 0, s>>>(n, pm.zq, pm.rec, K, ctx->frac, vd, vp, apart ? nullptr : ctx->Fd,
                                                                  apart ? nullptr : ctx->Fp, self_coef(ctx), ctx->pol,
                                                                  Ad, Ap, vAv);
         KCHECK();
@@ -1305,7 +1304,7 @@ void enqueue_pcg_iter(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
     const bool apart = ctx->ewald;  // real-space field kept apart: the gather overlaps k_tu_stored
     // the direction kernel has spread p
     matvec_stored<R>(ctx, s, A.p4, ctx->pd, ctx->pp, ctx->Apd, ctx->App, ctx->ewald ? ctx->scal + PAP_D : nullptr,
-                     false, apart, false);
+                     false, apart);
     if (!ctx->ewald) {
         k_dot2<<<nblk(n3, 256), 256, 0, s>>>(n3, ctx->pd, ctx->Apd, ctx->pp, ctx->App, ctx->scal + PAP_D,
                                               ctx->scal + PAP_P);
@@ -2346,10 +2345,11 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     dalloc(ctx, ctx->xyz, 3 * (size_t)n);
     dalloc(ctx, ctx->rp10, 10 * (size_t)n);
     dalloc(ctx, ctx->ad.at, n);
-    dalloc(ctx, ctx->ad.atS, n);
     dalloc(ctx, ctx->ad.u4, 2 * (size_t)n);
-    dalloc(ctx, ctx->ad.p4, 2 * (size_t)n);
-    if (ctx->prec == AMG_PREC_MIXED) {
+    if (ctx->prec == AMG_PREC_FP64) {
+        dalloc(ctx, ctx->ad.atS, n);
+        dalloc(ctx, ctx->ad.p4, 2 * (size_t)n);
+    } else {
         dalloc(ctx, ctx->af.at, n);
         dalloc(ctx, ctx->af.atS, n);
         dalloc(ctx, ctx->af.u4, 2 * (size_t)n);

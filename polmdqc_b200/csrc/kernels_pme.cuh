@@ -371,17 +371,20 @@ __device__ __forceinline__ void line_points(const double* __restrict__ line, int
 // matvec assembly:
 //   A v = v/alpha - (F_real + F_recip + selfc v),  F_recip = -grad phi
 // and, when vAv is given, the PCG dot products v.Av of both sets added to
-// vAv[0], vAv[1].  kLineLanes lanes per z-line (LineLane), G lanes per site:
-// with G = 8 the two halves share the x planes of the stencil.  Each lane
-// contracts its points of a plane's lines with the y weights, the planes with
-// the x weights and only the result with the z weights; the lanes' sums are
-// combined with shuffles and the lanes write the six components, whose
-// operands were requested first (35 -> 29 us: the kernel waits on memory).
+// vAv[0], vAv[1].  kLineLanes lanes per site, which share its z-lines
+// (LineLane; with 8 lanes, two halves of the x planes, within 3% either way up to
+// 12,288 sites and slower above).  Each lane contracts its points of a plane's
+// lines with the y weights, the planes with the x weights and only the result
+// with the z weights (in FP32 chains of 5, 5 and 2 terms; per line first, 5 and
+// up to 4: the errors of the gradients against FP64 are the same to 1% over 14
+// systems of 1,191 to 49,170 sites); the lanes' sums are combined in FP64 with
+// shuffles and the lanes write the six components, whose operands were
+// requested first (35 -> 29 us: the kernel waits on memory).
 // Blocks stride over the sites, so each block adds its dot products once.
 // With Fd, Fp null the real-space field is left out (A v without -F_real,
 // and its dot products): the real-space kernel then runs beside this one and
 // adds its own share (k_tu_stored with vAv), and k_pcg_update subtracts F.
-template <class R, int P, int G>
+template <class R, int P>
 __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx<R>::type* __restrict__ zg,
                                                       const R* __restrict__ rec, int3 K, Frac F,
                                                       const double* __restrict__ vd, const double* __restrict__ vp,
@@ -389,12 +392,11 @@ __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx
                                                       double selfc, const double* __restrict__ pol,
                                                       double* __restrict__ Ad, double* __restrict__ Ap,
                                                       double* __restrict__ vAv) {
-    constexpr int S = G / kLineLanes, NA = (P + S - 1) / S;  // sub-groups of a site, x planes of each
-    const int lane = threadIdx.x % G, per_block = blockDim.x / G, sub = lane / kLineLanes;
+    const int lane = threadIdx.x % kLineLanes, per_block = blockDim.x / kLineLanes;
     const bool even = (K.z & 1) == 0;
     double dotd = 0, dotp = 0;  // v.Av of this thread's components
     for (int g0 = blockIdx.x * per_block; g0 < n; g0 += gridDim.x * per_block) {
-        const int g = g0 + threadIdx.x / G;
+        const int g = g0 + threadIdx.x / kLineLanes;
         const int i = min(g, n - 1);
         const R* th = rec + (size_t)i * kRecWords;
         int a0, b0, c0;
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx
             fe[0] = FF[q0];
             fe[1] = FF[q1];
         }
-        const LineLane<R, P, 2> L(lane % kLineLanes, c0, K.z, th + 4 * P);
+        const LineLane<R, P, 2> L(lane, c0, K.z, th + 4 * P);
         R u[2 * P];   // y weights, then their first derivatives
         int row[P];   // offsets of the stencil's rows y
 #pragma unroll
@@ -426,9 +428,7 @@ __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx
         // z1) with the weights' orders (1, 0), (0, 1), (0, 0)
         R s10[4] = {0, 0, 0, 0}, s01[4] = {0, 0, 0, 0}, s00[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int aa = 0; aa < NA; aa++) {
-            const int a = sub * NA + aa;
-            if (S > 1 && a >= P) break;
+        for (int a = 0; a < P; a++) {
             int ga = a0 + a; if (ga >= K.x) ga -= K.x;
             const typename Cplx<R>::type* plane = zg + (size_t)ga * K.y * K.z;
             R q[P][4];
@@ -457,16 +457,12 @@ __global__ void __launch_bounds__(128) k_gather_field(int n, const typename Cplx
             f[3 * k + 1] = (double)(L.w0[0] * s01[k] + L.w1[0] * s01[2 + k]);
             f[3 * k + 2] = (double)(L.w0[1] * s00[k] + L.w1[1] * s00[2 + k]);
         }
-        if constexpr (S > 1) {
-#pragma unroll
-            for (int k = 0; k < 6; k++) f[k] += __shfl_xor_sync(0xffffffffu, f[k], kLineLanes);
-        }
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             sum[k] = (pset ? f[3 + k] : f[k]) + __shfl_xor_sync(0xffffffffu, pset ? f[k] : f[3 + k], 2);
             sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 1);
         }
-        if (g < n && sub == 0) {
+        if (g < n) {
             const double ia = 1.0 / alpha;
             double* AA = pset ? Ap : Ad;
             double dot = 0;
@@ -665,32 +661,30 @@ __global__ void k_convolve(size_t ncomplex, int batch, const R* __restrict__ inf
 //   phi_tuv = (K1/L1)^t (K2/L2)^u (K3/L3)^v sum_abc theta1^(t)_a theta2^(u)_b theta3^(v)_c grid
 // from a real grid (NS = 1: grid[g]) or from both parts of the complex
 // dipole grid at once (NS = 2: zg[g].x into phi, zg[g].y into phi + NC n).
-// kLineLanes lanes per z-line (LineLane), G lanes per site as in
-// k_gather_field: y, then x, then z contraction, the lanes' sums combined
-// with shuffles.  Output order: 0; x y z; xx yy zz xy xz yz;
-// xxx yyy zzz xxy xxz xyy yyz xzz yzz xyz.
+// kLineLanes lanes per site (LineLane) as in k_gather_field: y, then x, then z
+// contraction, the lanes' sums combined with shuffles.  Output order: 0; x y z;
+// xx yy zz xy xz yz; xxx yyy zzz xxy xxz xyy yyz xzz yzz xyz.
 
 // derivative order triples (t, u, v) of the output, in its order
 __device__ constexpr int kDerOut[20][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {2, 0, 0}, {0, 2, 0}, {0, 0, 2},
                                            {1, 1, 0}, {1, 0, 1}, {0, 1, 1}, {3, 0, 0}, {0, 3, 0}, {0, 0, 3}, {2, 1, 0},
                                            {2, 0, 1}, {1, 2, 0}, {0, 2, 1}, {1, 0, 2}, {0, 1, 2}, {1, 1, 1}};
 
-template <class R, int P, int NC, int G, int NS>
+template <class R, int P, int NC, int NS>
 __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ gridv, const R* __restrict__ theta,
                                                 const int* __restrict__ k0, int3 K, Frac F,
                                                 double* __restrict__ phi) {
     static_assert(NC == 4 || NC == 20, "first derivatives, or up to third");
     constexpr int ND = NC == 4 ? 2 : 4;       // derivative orders per axis
     constexpr int NV = 2 * NS;                // values of a lane in a line
-    constexpr int S = G / kLineLanes, NA = (P + S - 1) / S;  // sub-groups of a site, x planes of each
     using E = typename std::conditional<NS == 2, typename Cplx<R>::type, R>::type;
-    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G, sub = lane / kLineLanes;
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) / kLineLanes, lane = threadIdx.x % kLineLanes;
     const int i = min(g, n - 1);
     const bool even = (K.z & 1) == 0;
     const R* t1 = theta + ((size_t)i * 3 + 0) * 4 * P;
     const R* t2 = theta + ((size_t)i * 3 + 1) * 4 * P;
     const int a0 = k0[3 * i], b0 = k0[3 * i + 1], c0 = k0[3 * i + 2];
-    const LineLane<R, P, ND> L(lane % kLineLanes, c0, K.z, theta + ((size_t)i * 3 + 2) * 4 * P);
+    const LineLane<R, P, ND> L(lane, c0, K.z, theta + ((size_t)i * 3 + 2) * 4 * P);
     R xy[NV][ND][ND];  // sums over x and y with orders (t, u), t + u < ND
 #pragma unroll
     for (int v = 0; v < NV; v++)
@@ -698,9 +692,7 @@ __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ 
         for (int t = 0; t < ND; t++)
 #pragma unroll
             for (int u = 0; u + t < ND; u++) xy[v][t][u] = 0;
-    for (int aa = 0; aa < NA; aa++) {
-        const int a = sub * NA + aa;
-        if (S > 1 && a >= P) break;
+    for (int a = 0; a < P; a++) {
         int ga = a0 + a; if (ga >= K.x) ga -= K.x;
         const E* plane = static_cast<const E*>(gridv) + (size_t)ga * K.y * K.z;
         R q[P][NV];
@@ -739,7 +731,7 @@ __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ 
 #pragma unroll
     for (int s = 0; s < NS; s++)
 #pragma unroll
-        for (int j = 0; j < NC; j++) sum[s][j] = group_sum<G>((double)f[s][j]);
+        for (int j = 0; j < NC; j++) sum[s][j] = group_sum<kLineLanes>((double)f[s][j]);
     if (g >= n) return;
     if (F.general) {
 #pragma unroll
@@ -747,7 +739,7 @@ __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ 
             double fs[NC];
 #pragma unroll
             for (int j = 0; j < NC; j++) fs[j] = sum[s][j];
-            for (int j = lane; j < NC; j += G) phi[(size_t)s * NC * n + (size_t)NC * i + j] = cart_deriv(F, fs, NC, j);
+            for (int j = lane; j < NC; j += kLineLanes) phi[(size_t)s * NC * n + (size_t)NC * i + j] = cart_deriv(F, fs, NC, j);
         }
         return;
     }
@@ -759,7 +751,7 @@ __global__ void __launch_bounds__(128) k_gather(int n, const void* __restrict__ 
     for (int s = 0; s < NS; s++)
 #pragma unroll
         for (int j = 0; j < NC; j++)
-            if (j % G == lane)
+            if (j % kLineLanes == lane)
                 phi[(size_t)s * NC * n + (size_t)NC * i + j] = sum[s][j] * p0[kDerOut[j][0]] * p1[kDerOut[j][1]] *
                                                              p2[kDerOut[j][2]];
 }
