@@ -2850,7 +2850,7 @@ int amg_create(const amg_params* params, amg_ctx** out) {
     amg_ctx* ctx = new amg_ctx();
     try {
         rc = create_impl(ctx, params);
-        finish_setup(ctx);
+        if (rc == AMG_OK) finish_setup(ctx);
     } catch (Fail& f) {
         rc = f.code;
     }
