@@ -6,6 +6,9 @@
 // and joined to one.  Everything between amg_set_coords and the result copy
 // stays on the device; in a captured evaluation the PCG's last kernel decides
 // there whether the loop goes on.
+//
+// The times beside the choices below compare the two sides of a choice in one
+// tree and one way of measuring; those of different comments are not one series.
 #include "../../include/amoeba_gpu.h"
 #include "kernels_setup.cuh"
 #include "kernels_pme.cuh"
@@ -44,11 +47,13 @@ constexpr size_t kRbPiece = 16384;
 // From this many values the GPU takes over what the host does to a caller's
 // pinned arrays: it adds the gradients (the arrays' old values copied to the
 // device beside the solve, the sums straight back) and checks the coordinates.
-// The host's passes over arrays that are not in its caches run at ~10 GB/s (a
-// step with three contexts taking turns: 32,768 waters 3.78 -> 3.56 ms, 19,683
-// with direct polarization 0.98 -> 0.87, 13,824 without any 0.72 -> 0.68); with
-// 72,132 values the copies and the synchronisation cost 0.7% more than they
-// save (1.91 -> 1.92 ms).
+// The host's passes over arrays that are not in its caches run at ~10 GB/s.  Step
+// with three contexts taking turns, host / GPU: direct polarization, 24,696
+// values 245 / 250 us, 45,000 372 / 348, 72,000 508 / 449, 98,298 648 / 559,
+// 124,416 746 / 651; 32,768 waters with a solve 3.78 / 3.56 ms.  The line lies
+// above 72,132 values because there, with an FP64 solve that hides the host's
+// share, the copies and the synchronisation cost 0.7% (1.91 / 1.92 ms); without a
+// solve it could lie at half of that.
 constexpr size_t kGpuHostArrays = 98304;
 // FP64 accumulators (eacc): em real 0, einter 1, em reciprocal 2, net charge
 // 3, ep 4; the virial's six sums (xx yy zz xy xz yz) of em from kVir and of
@@ -881,11 +886,11 @@ void enqueue_lists(amg_ctx* ctx, cudaStream_t s) {
     size_t ncell = (size_t)cg.nc[0] * cg.nc[1] * cg.nc[2];
     double2* sdt = ctx->has_pol ? ctx->sdt : nullptr;
     // Ordered by counting where the cells are small (256 sites on average at
-    // most: a cell's ids are compared with one another) and few enough for the
-    // one block that scans them, else by a radix sort, which takes a few
-    // thousand sites in a single tile (evaluation by counting / radix sort: 648
-    // sites 358 / 355 us, 4,500: 518 / 518, 12,288: 766 / 786, 24,044 in FP64
-    // 1,767 / 1,811)
+    // most) and few enough for the one block that scans them, else by a radix
+    // sort, which takes a few thousand sites in a single tile.  Evaluation by
+    // radix sort / counting: 4,500 sites 470 / 469 us, 6,144: 531 to 546 / 540,
+    // 9,600: 627 to 647 / 636 (the sort's two values by where its arrays lie),
+    // 12,288: 721 / 689, 24,044 in FP64 1,811 / 1,767.
     if (n > 6144 && ncell <= 65536 && (size_t)n <= 256 * ncell) {
         int* slot = ctx->sids;  // the order's own array: free until it is written
         k_cell_count<<<nblk(n), kThreads, 0, s>>>(n, ctx->xyz, cg, ctx->bx, ctx->keys, slot, ctx->ccount);
@@ -1087,9 +1092,10 @@ double self_coef(const amg_ctx* ctx) {
 bool ewald_cells(const amg_ctx* ctx) { return ctx->ewald && ctx->bx.shape != 0; }
 
 // A v for both dipole sets (v/alpha - field of v), pair tensors computed on
-// the fly (FP64 correction sweep, OPT orders).  `cells` (the sweep, which
-// follows a solve and so has the cell-order partner rows cnb): the FP64
-// real-space part gathers from cell-order copies (k_Tu_cells).
+// the fly (OPT orders and their adjoint; a mixed context's FP64 sweep).
+// `cells` (the sweep, which follows a solve and so has the cell-order partner
+// rows cnb): the FP64 real-space part gathers from cell-order copies
+// (k_Tu_cells).
 template <class R>
 void matvec(amg_ctx* ctx, cudaStream_t s, const double* vd, const double* vp, double* Ad, double* Ap,
             bool cells = false, bool finish = true) {
@@ -1323,9 +1329,11 @@ void enqueue_pcg_iter(amg_ctx* ctx, cudaStream_t s, cudaGraphConditionalHandle h
 // FP64 correction sweep: the true residual with every term in FP64, one
 // diagonal-preconditioned step u += alpha r, and the residual norms.  An FP64
 // context has the FP64 coefficient rows of its solve (24,044 sites: 49 us
-// streamed against 75 computed on the fly).  With grad (the forward of
-// precision R) k_correct also prepares the force kernels' dipoles and
-// accumulators.
+// streamed against 75 computed on the fly, 1,909 against 1,988 us per step); a
+// bit of each coefficient holds a sign there, and the outputs equal those from
+// the pair geometry to 7e-16 of their norm (24,044 sites; 8e-16 at 8,232).  With
+// grad (the forward of precision R) k_correct also prepares the force kernels'
+// dipoles and accumulators.
 template <class R>
 void enqueue_sweep(amg_ctx* ctx, cudaStream_t s, bool forward, bool grad) {
     const int n = ctx->n;
@@ -2268,8 +2276,9 @@ int create_impl(amg_ctx* ctx, const amg_params* P) {
     }
     if (const char* g = getenv("AMG_NO_GRAPH")) ctx->use_graphs = !(g[0] == '1');
     // lanes per site of the bulk pair kernels: 8, or 16 where 8 leave the chip
-    // half empty and each lane a long serial share (evaluation with 8 / 16 / 32:
-    // 216 waters 402, 393, 402 us; 1,500: 539, 523, 528; 4,096: 782, 793, 814)
+    // half empty and each lane a long serial share (evaluation with 8 / 16: 648
+    // sites 402 / 393 us, 4,500: 494 / 470, 6,144: 541 / 541, 7,500: 552 / 550,
+    // 8,190: 558 / 561, 9,600: 632 / 632, 12,288: 686 / 697; 32 is slower than 16)
     ctx->lpa = n <= 8192 ? 16 : 8;
     if (const char* l = getenv("AMG_LPA")) ctx->lpa = atoi(l);
     if (ctx->lpa != 8 && ctx->lpa != 16 && ctx->lpa != 32) ctx->lpa = 16;
@@ -2616,8 +2625,10 @@ void adjoint_solve(amg_ctx* ctx, cudaStream_t s) {
     enqueue_sweep<R>(ctx, s, false, false);
 }
 
-// amg_backward: the adjoint solve in the context's precision (above), every
-// other term in FP64 (see kernels_adjoint.cuh for the algebra)
+// amg_backward: the adjoint solve in the context's precision (above), and in
+// that precision too the bulk pairs and the potentials of the dipole grids;
+// scaled pairs, OPT orders of the cotangents and everything per site in FP64
+// (see kernels_adjoint.cuh for the algebra)
 int backward_impl(amg_ctx* ctx, const amg_cotangents* cot, amg_param_grads* gr) {
     const int n = ctx->n;
     cudaStream_t s = ctx->st;
